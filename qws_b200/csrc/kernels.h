@@ -230,8 +230,6 @@ void spinor_h2h(const Geom& G, __half* dst, const __half* src, cudaStream_t st);
 // FP16 copies of the FP32 gauge (9 complex planes per mu) and clover planes
 void fields_s2h(const Geom& G, __half* Uh, const float* Us, __half* Ch, const float* Cs,
                 cudaStream_t st);
-// FP16 copy of per-RHS FP32 clover planes (entries of a multi-RHS handle)
-void clover_s2h_entries(const Geom& G, __half* Ch, const float* Cs, cudaStream_t st);
 // Device-side scalars of the flexible inner BiCGStab of one right-hand side
 // (bicgstab_precdd_s_h.cc:83-369): the loop's reductions land in res, a
 // one-thread kernel turns them into the next update's coefficients, kept

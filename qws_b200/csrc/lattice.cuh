@@ -628,6 +628,19 @@ struct IO<H16> {
       q[(size_t)j * pad + g] = make_uint4(x.x, x.y, y.x, y.y);
     }
   }
+  // one block's 36 reals
+  __device__ __forceinline__ static void store_clover_block(__half* C, int pad, int g, int blk,
+                                                            const float a[36]) {
+    uint4* q = reinterpret_cast<uint4*>(C);
+    const int first = blk ? 5 : 0, o = blk ? 4 : 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint2 x = pack4(a + o + 8 * j, 1.0f), y = pack4(a + o + 8 * j + 4, 1.0f);
+      q[(size_t)(first + j) * pad + g] = make_uint4(x.x, x.y, y.x, y.y);
+    }
+    reinterpret_cast<uint2*>(q + (size_t)4 * pad)[2 * (size_t)g + blk] =
+        pack4(a + (blk ? 0 : 32), 1.0f);
+  }
 };
 
 // FP16 spinors of a multi-RHS field computed two right-hand sides per

@@ -92,3 +92,33 @@ def test_device_gauge_matches_host():
     finally:
         host.close()
         dev.close()
+
+
+@pytest.mark.parametrize("shape, NB, csw", [
+    ((6, 3, 5, 2), (2, 1, 1, 2), 1.7),      # odd extents, extent 2, a ragged last block
+    ((18, 18, 22, 20), (2, 2, 2, 2), 1.7),  # walks of 4 sites, extents not multiples of 4
+    ((4, 4, 6, 8), (2, 1, 1, 1), 12.0),     # indefinite blocks: the pivoted inverse
+])
+def test_clover_operator_at_edges(shape, NB, csw):
+    """A^-1 on every site, FP64: A^-1 v of the device-built term against the
+    host generator's.  Both are backward-stable inverses of the same T, so
+    they differ by its condition number (below 1e3 but for rare sites of the
+    indefinite case) in FP64 roundoffs."""
+    import qws_b200
+
+    U, _ = qws_b200.gen_gauge(shape, 8, 5, 0.36)
+    C = qws_b200.gen_clover(U, shape, csw, KAPPA)
+    host = qws_b200.Lattice(shape, NB, tbc=-1, kappa=KAPPA)
+    dev = qws_b200.Lattice(shape, NB, tbc=-1, kappa=KAPPA)
+    try:
+        host.load_fields(U, C)
+        dev.load_gauge(U)
+        dev.build_clover(csw)
+        x = qws_b200.gen_source(shape, 9)
+        for p in (0, 1):
+            got = dev.to_host(dev.clv(dev.to_device(x), p))
+            want = host.to_host(host.clv(host.to_device(x), p))
+            assert rel(got, want) < (1e-13 if csw < 2 else 1e-10), p
+    finally:
+        host.close()
+        dev.close()
