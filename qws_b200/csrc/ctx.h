@@ -190,12 +190,31 @@ struct Ctx {
   const float* eoUs = nullptr;
   const float* eoCs = nullptr;
   int pce = 0, pco = 1;
-  double* eo_d[6] = {};
-  // multi-shift CG: the shifts' search vectors (ms_n fields back to back)
+  // compact one-parity copies of those fields (eo.cu), made on first use
+  // after every change of the fields they were made from, and work vectors
+  // of one parity each (24 * eo_pad() reals)
+  double* eoc_Ud = nullptr;
+  double* eoc_Cd = nullptr;
+  float* eoc_Us = nullptr;
+  float* eoc_Cs = nullptr;
+  // which state of the fields they were made from: every change of the
+  // fields of a handle gives it a new number (unique in the process, so that
+  // a borrowing handle sees its parent's changes and a change of parent)
+  long fields_gen_d = next_fields_gen(), fields_gen_s = next_fields_gen();
+  long eoc_gen_d = 0, eoc_gen_s = 0;
+  static long next_fields_gen();
+  int eo_pad() const { return (G.Vh + 127) / 128 * 128; }
+  static constexpr int kEoVecs = 9;
+  double* eo_d[kEoVecs] = {};
+  float* eo_s[3] = {};
+  // multi-shift CG: the shifts' search vectors and solutions (ms_n compact
+  // vectors each, back to back)
   double* ms_p = nullptr;
+  double* ms_x = nullptr;
   int ms_n = 0;
-  float* eo_s[2] = {};
-  void ensure_eo();
+  // the compact fields and the first n work vectors
+  void ensure_eo_d(int n);
+  void ensure_eo_s(int n);
   long n_mtilde = 0;
 
   // CUDA graphs of the SAP preconditioner's launch sequences (about 40

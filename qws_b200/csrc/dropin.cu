@@ -195,6 +195,8 @@ void sync_eo(Ctx& c) {
     qws_to_planes_clover<float>(c.G, g.eCs, (const float*)d, g.vlens, c.st, true);
     c.check_launch("even-odd field upload");
     QWSG_CUDA(cudaStreamSynchronize(c.st));
+    c.fields_gen_d = Ctx::next_fields_gen();
+    c.fields_gen_s = Ctx::next_fields_gen();
     g.eo_dirty = false;
   }
   c.eoUd = g.eUd;

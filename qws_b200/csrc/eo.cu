@@ -1,6 +1,6 @@
 // Even-odd (site parity) hopping kernels: the deo_* family of the reference
 // (deo_in_d.cc:65-445, deo_out_d.cc:88-286, deo_dag_in.cc, deo_dag_out.cc and
-// the FP32 deo_in_s.cc / deo_out_s.cc) on the library's DD-order planes.
+// the FP32 deo_in_s.cc / deo_out_s.cc).
 //
 // Sites of parity pe = (x+y+z+t) % 2 receive the hops from the other parity:
 //   WHICH  1 = hops inside the rank box (deo_in_*), 2 = hops across its faces
@@ -10,8 +10,18 @@
 //   CLOV   multiply by the parity's A^-1 (dee_*);
 //   MODE   0 out = acc (__store_sc), 1 out += coef acc (__store_add_sc),
 //          2 out = in0 + coef acc (one_minus_*).
-// A y/z/t hop that leaves the rank box reads the other parity's site at the
-// same compressed index x/2 of the wrapped row, as the reference's face
+//
+// The operators work on vectors and fields of one parity each, stored
+// compactly in the order e = x/2 + Lx/2 (y + Ly (z + Lz t)).  On the full
+// lattice's planes the two parities alternate along a row, so one parity's
+// 16-byte entries use half of every 32-byte sector; compact, every byte
+// fetched is used (FP64 normal operator at 24^3x48: 2.6 ms on full planes
+// walked in x order, 0.70 ms compact).  Full-plane vectors of
+// the API are gathered and scattered by eo_gather / eo_scatter, the fields
+// once per load.
+//
+// A y/z/t hop reads the other parity's site at the same compressed index x/2
+// of the neighbouring row, also across a boundary, as the reference's face
 // packers do (deo_out_d.cc:88-153); this is the geometric neighbour when the
 // wrapped extent is even.
 #include "kernels.h"
@@ -19,27 +29,58 @@
 
 namespace qwsg {
 
+// compact index of the site with coordinates x, within its parity
+__device__ __forceinline__ int eo_index(const Geom& G, const int x[4]) {
+  return (x[0] >> 1) + (G.L[0] >> 1) * (x[1] + G.L[1] * (x[2] + G.L[2] * x[3]));
+}
+
+struct EoSite {
+  int xh, y, z, t;
+  int odd;  // x = 2 xh + odd
+};
+template <typename T>
+__device__ __forceinline__ EoSite eo_site(const EoArgs<T>& a, int e) {
+  EoSite s;
+  int k = fdiv(e, a.dxh);
+  s.xh = e - k * (a.G.L[0] >> 1);
+  int q = fdiv(k, a.dy);
+  s.y = k - q * a.G.L[1];
+  s.t = fdiv(q, a.dz);
+  s.z = q - s.t * a.G.L[2];
+  s.odd = (a.pe + s.y + s.z + s.t) & 1;
+  return s;
+}
+
 template <typename T, int WHICH, int DAG, int MU, int DIR, typename R = typename Arith<T>::R>
-__device__ __forceinline__ void eo_hop(const EoArgs<T>& a, const int x[4], int g, R acc[24]) {
-  const int L = a.G.L[MU], box = a.box[MU];
-  const bool inner = DIR > 0 ? (x[MU] % box) != box - 1 : (x[MU] % box) != 0;
-  if (inner ? !(WHICH & 1) : !(WHICH & 2)) return;
-  int xn[4] = {x[0], x[1], x[2], x[3]};
-  xn[MU] = DIR > 0 ? (x[MU] + 1 == L ? 0 : x[MU] + 1) : (x[MU] == 0 ? L - 1 : x[MU] - 1);
-  if (!inner && MU > 0) {
-    const int po = 1 - ((x[0] + x[1] + x[2] + x[3]) & 1);
-    xn[0] = 2 * (x[0] >> 1) + ((po + xn[1] + xn[2] + xn[3]) & 1);
+__device__ __forceinline__ void eo_hop(const EoArgs<T>& a, const EoSite& s, int e, R acc[24]) {
+  const int nxh = a.G.L[0] >> 1;
+  const int c = MU == 0 ? 2 * s.xh + s.odd : MU == 1 ? s.y : MU == 2 ? s.z : s.t;
+  if (WHICH != 3) {
+    const int box = a.box[MU], in_box = c % box;
+    const bool inner = DIR > 0 ? in_box != box - 1 : in_box != 0;
+    if (inner ? !(WHICH & 1) : !(WHICH & 2)) return;
   }
-  const int gn = dd_index(a.G, xn);
+  int en = e;
+  if (MU == 0) {
+    // x+1 of an even x and x-1 of an odd x have the same compressed index
+    if (DIR > 0 && s.odd) en = s.xh + 1 == nxh ? e - (nxh - 1) : e + 1;
+    if (DIR < 0 && !s.odd) en = s.xh == 0 ? e + (nxh - 1) : e - 1;
+  } else {
+    const int str = MU == 1 ? nxh : MU == 2 ? nxh * a.G.L[1] : nxh * a.G.L[1] * a.G.L[2];
+    const int L = a.G.L[MU];
+    en = DIR > 0 ? (c + 1 == L ? e - (L - 1) * str : e + str)
+                 : (c == 0 ? e + (L - 1) * str : e - str);
+  }
   constexpr int PD = DAG ? -DIR : DIR;  // projector / reconstruction of this hop
   R v[24];
   if (MU == 3)
-    IO<T>::load_half(a.src, a.G.pad, gn, PD > 0, v);
+    IO<T>::load_half(a.src, a.pad, en, PD > 0, v);
   else
-    IO<T>::load_spinor(a.src, a.G.pad, gn, v);
+    IO<T>::load_spinor(a.src, a.pad, en, v);
   R h[12], r[12], u[18];
   project<R, MU, PD>(v, h);
-  IO<T>::load_link(a.U, a.G.pad, MU, DIR > 0 ? g : gn, u);
+  // forward: this parity's own link, backward: the other parity's
+  IO<T>::load_link(DIR > 0 ? a.U[0] : a.U[1], a.pad, MU, DIR > 0 ? e : en, u);
   if (DIR > 0)
     link_mul<R, false>(u, h, r);
   else
@@ -47,105 +88,184 @@ __device__ __forceinline__ void eo_hop(const EoArgs<T>& a, const int x[4], int g
   R f = 1;
   if (MU == 3) {
     f = 2;
-    if (DIR > 0 ? x[3] == L - 1 : x[3] == 0) f = (R)(2 * a.G.tbc);
+    if (DIR > 0 ? s.t == a.G.L[3] - 1 : s.t == 0) f = (R)(2 * a.G.tbc);
   }
   reconstruct<R, MU, PD>(r, acc, f);
 }
 
+// Memory bound: per output site 8 links (1152 bytes in FP64, each link of the
+// lattice once per launch), A^-1, the source once and the result: 2112 bytes
+// in FP64, 118 us at 24^3x48, 0.91 of the measured copy rate.
 template <typename T, int WHICH, int DAG, int CLOV, int MODE>
-__global__ void __launch_bounds__(128) k_eo(const EoArgs<T> a) {
+__device__ __forceinline__ void eo_body(const EoArgs<T>& a) {
   using R = typename Arith<T>::R;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.G.Vh) return;
-  const int nxh = a.G.L[0] >> 1;
-  int x[4];
-  const int xh = i % nxh;
-  int k = i / nxh;
-  x[1] = k % a.G.L[1];
-  k /= a.G.L[1];
-  x[2] = k % a.G.L[2];
-  x[3] = k / a.G.L[2];
-  x[0] = 2 * xh + ((a.pe + x[1] + x[2] + x[3]) & 1);
-  const int g = dd_index(a.G, x);
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= a.G.Vh) return;
+  const EoSite s = eo_site(a, e);
   R acc[24];
 #pragma unroll
   for (int j = 0; j < 24; j++) acc[j] = 0;
-  eo_hop<T, WHICH, DAG, 0, +1>(a, x, g, acc);
-  eo_hop<T, WHICH, DAG, 0, -1>(a, x, g, acc);
-  eo_hop<T, WHICH, DAG, 1, +1>(a, x, g, acc);
-  eo_hop<T, WHICH, DAG, 1, -1>(a, x, g, acc);
-  eo_hop<T, WHICH, DAG, 2, +1>(a, x, g, acc);
-  eo_hop<T, WHICH, DAG, 2, -1>(a, x, g, acc);
-  eo_hop<T, WHICH, DAG, 3, +1>(a, x, g, acc);
-  eo_hop<T, WHICH, DAG, 3, -1>(a, x, g, acc);
-  if (CLOV) clover_apply<T>(a.C, a.G.pad, g, acc);
-  R o[24];
-  if (MODE == 0) {
+  eo_hop<T, WHICH, DAG, 0, +1>(a, s, e, acc);
+  eo_hop<T, WHICH, DAG, 0, -1>(a, s, e, acc);
+  eo_hop<T, WHICH, DAG, 1, +1>(a, s, e, acc);
+  eo_hop<T, WHICH, DAG, 1, -1>(a, s, e, acc);
+  eo_hop<T, WHICH, DAG, 2, +1>(a, s, e, acc);
+  eo_hop<T, WHICH, DAG, 2, -1>(a, s, e, acc);
+  eo_hop<T, WHICH, DAG, 3, +1>(a, s, e, acc);
+  eo_hop<T, WHICH, DAG, 3, -1>(a, s, e, acc);
+  if (CLOV) clover_apply<T>(a.C, a.pad, e, acc);
+  if (MODE == 2) {
+    R o[24];
+    IO<T>::load_spinor(a.in0, a.pad, e, o);
 #pragma unroll
-    for (int j = 0; j < 24; j++) o[j] = acc[j];
-  } else if (MODE == 1) {
-    IO<T>::load_spinor(a.out, a.G.pad, g, o);
-#pragma unroll
-    for (int j = 0; j < 24; j++) o[j] = o[j] + acc[j] * a.coef;
-  } else {
-    IO<T>::load_spinor(a.in0, a.G.pad, g, o);
-#pragma unroll
-    for (int j = 0; j < 24; j++) o[j] = o[j] + acc[j] * a.coef;
+    for (int j = 0; j < 24; j++) acc[j] = o[j] + acc[j] * a.coef;
   }
-  IO<T>::store_spinor(a.out, a.G.pad, g, o);
+  IO<T>::store_spinor(a.out, a.pad, e, acc);
+}
+// FP64 at 128 registers (4 CTAs of 128 threads an SM), FP32 at 80 (6)
+template <typename T, int WHICH, int DAG, int CLOV, int MODE>
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) k_eo(const EoArgs<T> a) {
+  eo_body<T, WHICH, DAG, CLOV, MODE>(a);
 }
 
-// parity-pe clover multiplication (clvd_vm_/clv_s_, qws.cc:390-425)
+// out = A^-1 in on compact vectors (as an epilogue of the operator before it,
+// a second A^-1 in one kernel spilled: 76 us against 25 + 11 at 16^3x32)
 template <typename T>
-__global__ void k_clv(const EoArgs<T> a) {
+__global__ void __launch_bounds__(128) k_eo_clv(const EoArgs<T> a) {
   using R = typename Arith<T>::R;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.G.Vh) return;
-  const int nxh = a.G.L[0] >> 1;
-  int x[4];
-  const int xh = i % nxh;
-  int k = i / nxh;
-  x[1] = k % a.G.L[1];
-  k /= a.G.L[1];
-  x[2] = k % a.G.L[2];
-  x[3] = k / a.G.L[2];
-  x[0] = 2 * xh + ((a.pe + x[1] + x[2] + x[3]) & 1);
-  const int g = dd_index(a.G, x);
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= a.G.Vh) return;
   R v[24];
-  IO<T>::load_spinor(a.src, a.G.pad, g, v);
-  clover_apply<T>(a.C, a.G.pad, g, v);
-  IO<T>::store_spinor(a.out, a.G.pad, g, v);
+  IO<T>::load_spinor(a.src, a.pad, e, v);
+  clover_apply<T>(a.C, a.pad, e, v);
+  IO<T>::store_spinor(a.out, a.pad, e, v);
 }
 
+// parity-pe clover multiplication on full planes (clvd_vm_/clv_s_,
+// qws.cc:390-425), walked in the planes' order
 template <typename T>
-__global__ void k_parity_select(Geom G, typename Store<T>::type* dst,
-                                const typename Store<T>::type* __restrict__ src, int pe) {
-  using R = typename Arith<T>::R;
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128) k_clv(Geom G, T* out, const T* __restrict__ in,
+                                             const T* __restrict__ C, int pe) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= G.V) return;
-  Site s;
-  decode_site(G, g, s);
-  int par = 0;
+  int x[4];
+  site_coords(G, g, x);
+  if (((x[0] + x[1] + x[2] + x[3]) & 1) != pe) return;
+  T v[24];
+  IO<T>::load_spinor(in, G.pad, g, v);
+  clover_apply<T>(C, G.pad, g, v);
+  IO<T>::store_spinor(out, G.pad, g, v);
+}
+
+// full planes -> compact vector of parity pe.  Walked in the planes' order:
+// reads are runs, each write is a sector that its neighbour's write completes
+// in L2.
+template <typename T>
+__global__ void __launch_bounds__(128) k_eo_gather(Geom G, T* __restrict__ dst, int pad,
+                                                   const T* __restrict__ src, int pe) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= G.V) return;
+  int x[4];
+  site_coords(G, g, x);
+  if (((x[0] + x[1] + x[2] + x[3]) & 1) != pe) return;
+  T v[24];
+  IO<T>::load_spinor(src, G.pad, g, v);
+  IO<T>::store_spinor(dst, pad, eo_index(G, x), v);
+}
+// compact vector -> parity pe of full planes: MODE 0 out = v, 1 out += coef v,
+// 2 out = in0 + coef v; ZERO: the other parity becomes zero (else untouched)
+template <typename T, int MODE, bool ZERO>
+__global__ void __launch_bounds__(128) k_eo_scatter(Geom G, T* out, const T* __restrict__ v, int pad,
+                                                    const T* in0, T coef, int pe) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= G.V) return;
+  int x[4];
+  site_coords(G, g, x);
+  T o[24];
+  if (((x[0] + x[1] + x[2] + x[3]) & 1) != pe) {
+    if (!ZERO) return;
 #pragma unroll
-  for (int mu = 0; mu < 4; mu++) par += s.bc[mu] * G.B[mu] + s.lc[mu];
-  R v[24];
-  if ((par & 1) == pe) {
-    IO<T>::load_spinor(src, G.pad, g, v);
+    for (int j = 0; j < 24; j++) o[j] = 0;
   } else {
+    T a[24];
+    IO<T>::load_spinor(v, pad, eo_index(G, x), a);
+    if (MODE == 0) {
 #pragma unroll
-    for (int j = 0; j < 24; j++) v[j] = 0;
+      for (int j = 0; j < 24; j++) o[j] = a[j];
+    } else {
+      IO<T>::load_spinor(MODE == 1 ? out : in0, G.pad, g, o);
+#pragma unroll
+      for (int j = 0; j < 24; j++) o[j] = o[j] + a[j] * coef;
+    }
   }
-  IO<T>::store_spinor(dst, G.pad, g, v);
+  IO<T>::store_spinor(out, G.pad, g, o);
+}
+
+// full field planes -> the two parities' compact planes (parity p at
+// p * 72 * pad reals)
+template <typename T>
+__global__ void __launch_bounds__(128) k_eo_links(Geom G, T* __restrict__ dst, int pad,
+                                                  const T* __restrict__ U) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= G.V) return;
+  int x[4];
+  site_coords(G, g, x);
+  const int p = (x[0] + x[1] + x[2] + x[3]) & 1, e = eo_index(G, x);
+  T u[18];
+  IO<T>::load_link(U, G.pad, blockIdx.y, g, u);
+  store_link<T>(dst + (size_t)72 * pad * p, pad, blockIdx.y, e, u);
+}
+template <typename T>
+__global__ void __launch_bounds__(128) k_eo_clover(Geom G, T* __restrict__ dst, int pad,
+                                                   const T* __restrict__ C) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= G.V) return;
+  int x[4];
+  site_coords(G, g, x);
+  const int p = (x[0] + x[1] + x[2] + x[3]) & 1, e = eo_index(G, x);
+  T a[72];
+  IO<T>::load_clover_block(C, G.pad, g, 0, a);
+  IO<T>::load_clover_block(C, G.pad, g, 1, a + 36);
+  store_clover<T>(dst + (size_t)72 * pad * p, pad, e, a);
 }
 
 template <typename T>
-void parity_select(const Geom& G, typename Store<T>::type* dst, const typename Store<T>::type* src,
-                   int pe, cudaStream_t st) {
+void eo_fields(const Geom& G, T* Ue, T* Ce, int pad, const T* U, const T* C, cudaStream_t st) {
+  const int nb = (G.V + 127) / 128;
   count_launch();
-  k_parity_select<T><<<(G.V + 127) / 128, 128, 0, st>>>(G, dst, src, pe);
+  k_eo_links<T><<<dim3(nb, 4), 128, 0, st>>>(G, Ue, pad, U);
+  count_launch();
+  k_eo_clover<T><<<nb, 128, 0, st>>>(G, Ce, pad, C);
 }
-template void parity_select<float>(const Geom&, float*, const float*, int, cudaStream_t);
-template void parity_select<double>(const Geom&, double*, const double*, int, cudaStream_t);
+template <typename T>
+void eo_gather(const Geom& G, T* dst, int pad, const T* src, int pe, cudaStream_t st) {
+  count_launch();
+  k_eo_gather<T><<<(G.V + 127) / 128, 128, 0, st>>>(G, dst, pad, src, pe);
+}
+template <typename T>
+void eo_scatter(const Geom& G, T* out, const T* v, int pad, int pe, int mode, T coef, const T* in0,
+                bool zero_other, cudaStream_t st) {
+  const int nb = (G.V + 127) / 128;
+  count_launch();
+  if (mode == 1)
+    k_eo_scatter<T, 1, false><<<nb, 128, 0, st>>>(G, out, v, pad, in0, coef, pe);
+  else if (mode == 2)
+    k_eo_scatter<T, 2, false><<<nb, 128, 0, st>>>(G, out, v, pad, in0, coef, pe);
+  else if (zero_other)
+    k_eo_scatter<T, 0, true><<<nb, 128, 0, st>>>(G, out, v, pad, in0, coef, pe);
+  else
+    k_eo_scatter<T, 0, false><<<nb, 128, 0, st>>>(G, out, v, pad, in0, coef, pe);
+}
+template <typename T>
+void launch_clv(const Geom& G, T* out, const T* in, const T* C, int pe, cudaStream_t st) {
+  count_launch();
+  k_clv<T><<<(G.V + 127) / 128, 128, 0, st>>>(G, out, in, C, pe);
+}
+template <typename T>
+void launch_eo_clv(const EoArgs<T>& a, cudaStream_t st) {
+  count_launch();
+  k_eo_clv<T><<<(a.G.Vh + 127) / 128, 128, 0, st>>>(a);
+}
 
 template <typename T, int WHICH, int DAG, int CLOV, int MODE>
 static void go(const EoArgs<T>& a, cudaStream_t st) {
@@ -153,32 +273,32 @@ static void go(const EoArgs<T>& a, cudaStream_t st) {
   k_eo<T, WHICH, DAG, CLOV, MODE><<<(a.G.Vh + 127) / 128, 128, 0, st>>>(a);
 }
 
+// compact vectors: mode 0, or 2 for the two forms of the Schur operators
 template <typename T>
 void launch_eo(int which, int dag, int clov, int mode, const EoArgs<T>& a, cudaStream_t st) {
-  // every combination the reference uses (12 FP64, 5 FP32 entry points)
 #define QWSG_EO(W, D, C, M)                                    \
   if (which == W && dag == D && clov == C && mode == M) {      \
     go<T, W, D, C, M>(a, st);                                  \
     return;                                                    \
   }
   QWSG_EO(1, 0, 0, 0) QWSG_EO(1, 0, 1, 0) QWSG_EO(1, 1, 0, 0) QWSG_EO(1, 1, 1, 0)
-  QWSG_EO(1, 0, 1, 2) QWSG_EO(1, 1, 0, 2)
-  QWSG_EO(2, 0, 0, 1) QWSG_EO(2, 1, 0, 1) QWSG_EO(2, 0, 1, 1) QWSG_EO(2, 1, 1, 1)
+  QWSG_EO(2, 0, 0, 0) QWSG_EO(2, 0, 1, 0) QWSG_EO(2, 1, 0, 0) QWSG_EO(2, 1, 1, 0)
   QWSG_EO(3, 0, 0, 0) QWSG_EO(3, 0, 1, 0) QWSG_EO(3, 1, 0, 0) QWSG_EO(3, 1, 1, 0)
-  QWSG_EO(3, 0, 1, 2) QWSG_EO(3, 1, 0, 2) QWSG_EO(3, 0, 0, 1) QWSG_EO(3, 0, 1, 1)
+  QWSG_EO(3, 0, 1, 2) QWSG_EO(3, 1, 0, 2)
 #undef QWSG_EO
   throw_unsupported_eo();
 }
 
-template <typename T>
-void launch_clv(const EoArgs<T>& a, cudaStream_t st) {
-  count_launch();
-  k_clv<T><<<(a.G.Vh + 127) / 128, 128, 0, st>>>(a);
-}
-
-template void launch_eo<float>(int, int, int, int, const EoArgs<float>&, cudaStream_t);
-template void launch_eo<double>(int, int, int, int, const EoArgs<double>&, cudaStream_t);
-template void launch_clv<float>(const EoArgs<float>&, cudaStream_t);
-template void launch_clv<double>(const EoArgs<double>&, cudaStream_t);
+#define QWSG_INST(T)                                                                          \
+  template void launch_eo<T>(int, int, int, int, const EoArgs<T>&, cudaStream_t);             \
+  template void launch_eo_clv<T>(const EoArgs<T>&, cudaStream_t);                             \
+  template void launch_clv<T>(const Geom&, T*, const T*, const T*, int, cudaStream_t);        \
+  template void eo_fields<T>(const Geom&, T*, T*, int, const T*, const T*, cudaStream_t);     \
+  template void eo_gather<T>(const Geom&, T*, int, const T*, int, cudaStream_t);              \
+  template void eo_scatter<T>(const Geom&, T*, const T*, int, int, int, T, const T*, bool,    \
+                              cudaStream_t);
+QWSG_INST(float)
+QWSG_INST(double)
+#undef QWSG_INST
 
 }  // namespace qwsg

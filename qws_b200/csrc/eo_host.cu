@@ -1,11 +1,12 @@
 // Host side of the even-odd (site parity) operator family and its solver
 // (deo_*/dee_*/one_minus_*, clvd_vm_/clv_s_, mtilde_vm_, mtilde_dag_vm_,
 // mtilde_s_ of qws.cc:390-605 and bicgstab_vm_ of bicgstab.cc:68-333).
-// Parity fields live in the library's DD-order planes; a parity-p vector is
-// a full field whose other-parity sites are zero.
+// At the API a parity-p vector is the parity-p sites of full DD-order planes;
+// the operators and solvers here run on compact one-parity vectors (eo.cu).
 #include <cmath>
 #include <complex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "ctx.h"
@@ -16,33 +17,114 @@ namespace qwsg {
   throw Error(2, "even-odd operator: unsupported combination of hop set / adjoint / clover / mode");
 }
 
-void Ctx::ensure_eo() {
-  // each buffer on its own (a failed allocation is retried by the next call)
-  for (int i = 0; i < 6; i++)
-    if (!eo_d[i]) eo_d[i] = alloc_spinor<double>();
-  for (int i = 0; i < 2; i++)
-    if (!eo_s[i]) eo_s[i] = alloc_spinor<float>();
+// each buffer on its own (a failed allocation is retried by the next call)
+template <typename R>
+static void eo_alloc(Ctx& c, R** p, size_t n) {
+  if (*p) return;
+  void* q = nullptr;
+  QWSG_CUDA(cudaMalloc(&q, sizeof(R) * n));
+  c.owned.push_back(q);
+  *p = static_cast<R*>(q);
+  QWSG_CUDA(cudaMemsetAsync(q, 0, sizeof(R) * n, c.st));
+}
+template <typename R>
+static void eo_ensure(Ctx& c, R** U, R** C, long& made, long gen, const R* srcU, const R* srcC,
+                      R** vecs, int n) {
+  if (!srcU || !srcC) throw Error(4, "gauge/clover fields not loaded");
+  const size_t pad = c.eo_pad();
+  eo_alloc(c, U, 144 * pad);
+  eo_alloc(c, C, 144 * pad);
+  for (int i = 0; i < n; i++) eo_alloc(c, vecs + i, 24 * pad);
+  if (made == gen) return;
+  eo_fields<R>(c.G, *U, *C, (int)pad, srcU, srcC, c.st);
+  c.check_launch("eo_fields");
+  made = gen;
+}
+void Ctx::ensure_eo_d(int n) {
+  eo_ensure<double>(*this, &eoc_Ud, &eoc_Cd, eoc_gen_d, (parent ? parent : this)->fields_gen_d,
+                    eoUd ? eoUd : Ud, eoCd ? eoCd : Cd, eo_d, n);
+}
+void Ctx::ensure_eo_s(int n) {
+  eo_ensure<float>(*this, &eoc_Us, &eoc_Cs, eoc_gen_s, (parent ? parent : this)->fields_gen_s,
+                   eoUs ? eoUs : Us, eoCs ? eoCs : Cs, eo_s, n);
 }
 
 template <typename R>
-static EoArgs<R> eo_args(Ctx& c, int pe);
-template <>
-EoArgs<double> eo_args<double>(Ctx& c, int pe) {
-  EoArgs<double> a{};
+static bool eo_loaded(const Ctx& c) {
+  if constexpr (std::is_same<R, double>::value)
+    return (c.eoUd || c.Ud) && (c.eoCd || c.Cd);
+  else
+    return (c.eoUs || c.Us) && (c.eoCs || c.Cs);
+}
+
+// the compact vectors as the BLAS kernels see them: one RHS of Vh sites
+static Geom eo_geom(const Ctx& c) {
+  Geom G = c.G;
+  G.V = c.G.Vh;
+  G.pad = c.eo_pad();
+  return G;
+}
+
+template <typename R>
+static EoArgs<R> eo_args(Ctx& c, int pe) {
+  EoArgs<R> a{};
   a.G = c.G;
-  a.U = c.eoUd ? c.eoUd : c.Ud;
-  a.C = c.eoCd ? c.eoCd : c.Cd;
+  a.pad = c.eo_pad();
+  const R *U, *C;
+  if constexpr (std::is_same<R, double>::value) {
+    U = c.eoc_Ud;
+    C = c.eoc_Cd;
+  } else {
+    U = c.eoc_Us;
+    C = c.eoc_Cs;
+  }
+  const size_t par = (size_t)72 * a.pad;
+  a.U[0] = U + pe * par;
+  a.U[1] = U + (1 - pe) * par;
+  a.C = C + pe * par;
   a.pe = pe;
+  // the reference's rank box: each rank holds two x-halves (NB = 2*npe0, ...)
+  a.box[0] = c.G.L[0] / (c.G.NB[0] / 2);
+  for (int mu = 1; mu < 4; mu++) a.box[mu] = c.G.L[mu] / c.G.NB[mu];
+  a.dxh = make_fastdiv(c.G.L[0] / 2);
+  a.dy = make_fastdiv(c.G.L[1]);
+  a.dz = make_fastdiv(c.G.L[2]);
   return a;
 }
-template <>
-EoArgs<float> eo_args<float>(Ctx& c, int pe) {
-  EoArgs<float> a{};
-  a.G = c.G;
-  a.U = c.eoUs ? c.eoUs : c.Us;
-  a.C = c.eoCs ? c.eoCs : c.Cs;
-  a.pe = pe;
-  return a;
+
+// one application on compact vectors (out: parity pe, in: the other; mode 0,
+// or 2: out = in0 + factor * hops)
+template <typename R>
+static void eo_apply(Ctx& c, R* out, const R* in, int pe, int which, int dag, int clov, int mode,
+                     double factor, const R* in0) {
+  auto a = eo_args<R>(c, pe);
+  a.src = in;
+  a.out = out;
+  a.in0 = in0;
+  a.coef = (R)factor;
+  launch_eo<R>(which, dag, clov, mode, a, c.st);
+}
+
+template <typename R>
+static R** eo_vecs(Ctx& c, int n) {
+  if constexpr (std::is_same<R, double>::value) {
+    c.ensure_eo_d(n);
+    return c.eo_d;
+  } else {
+    c.ensure_eo_s(n);
+    return c.eo_s;
+  }
+}
+
+// every combination the reference uses (12 FP64, 5 FP32 entry points)
+static bool eo_supported(int which, int dag, int clov, int mode) {
+  if (dag < 0 || dag > 1 || clov < 0 || clov > 1) return false;
+  switch (which) {
+    case 1: return mode == 0 || (mode == 2 && dag != clov);
+    case 2: return mode == 1;
+    case 3: return mode == 0 || (mode == 2 && dag != clov) || (mode == 1 && dag == 0);
+  }
+  return false;
 }
 
 template <typename R>
@@ -50,16 +132,14 @@ void deo(Ctx& c, R* out, const R* in, int pe, int which, int dag, int clov, int 
          double factor, const R* in0) {
   if (pe != 0 && pe != 1) throw Error(1, "parity must be 0 or 1");
   if (mode == 2 && !in0) throw Error(1, "mode 2 needs in0");
-  auto a = eo_args<R>(c, pe);
-  if (!a.U || !a.C) throw Error(4, "gauge/clover fields not loaded");
-  a.src = in;
-  a.out = out;
-  a.in0 = in0;
-  a.coef = (R)factor;
-  // the reference's rank box: each rank holds two x-halves (NB = 2*npe0, ...)
-  a.box[0] = c.G.L[0] / (c.G.NB[0] / 2);
-  for (int mu = 1; mu < 4; mu++) a.box[mu] = c.G.L[mu] / c.G.NB[mu];
-  launch_eo<R>(which, dag, clov, mode, a, c.st);
+  if (!eo_supported(which, dag, clov, mode)) {
+    if (!eo_loaded<R>(c)) throw Error(4, "gauge/clover fields not loaded");
+    throw_unsupported_eo();
+  }
+  R** v = eo_vecs<R>(c, 2);
+  eo_gather<R>(c.G, v[0], c.eo_pad(), in, 1 - pe, c.st);
+  eo_apply<R>(c, v[1], v[0], pe, which, dag, clov, 0, 0.0, nullptr);
+  eo_scatter<R>(c.G, out, v[1], c.eo_pad(), pe, mode, (R)factor, in0, false, c.st);
   c.check_launch("deo");
 }
 template void deo<float>(Ctx&, float*, const float*, int, int, int, int, int, double, const float*);
@@ -68,69 +148,91 @@ template void deo<double>(Ctx&, double*, const double*, int, int, int, int, int,
 
 template <typename R>
 void clv(Ctx& c, R* out, const R* in, int pe) {
-  auto a = eo_args<R>(c, pe);
-  if (!a.C) throw Error(4, "clover field not loaded");
-  a.src = in;
-  a.out = out;
-  launch_clv<R>(a, c.st);
+  const R* C;
+  if constexpr (std::is_same<R, double>::value)
+    C = c.eoCd ? c.eoCd : c.Cd;
+  else
+    C = c.eoCs ? c.eoCs : c.Cs;
+  if (!C) throw Error(4, "clover field not loaded");
+  launch_clv<R>(c.G, out, in, C, pe, c.st);
   c.check_launch("clv");
 }
 template void clv<float>(Ctx&, float*, const float*, int);
 template void clv<double>(Ctx&, double*, const double*, int);
 
 // mtilde_vm_: out_e = in_e - kappa^2 A_ee^-1 H_eo A_oo^-1 H_oe in_e
-// (dee_deo_vm_(pco, pce) then one_minus_dee_deo_vm_(pce, pco))
-void mtilde_d(Ctx& c, double* out, const double* in) {
-  c.ensure_eo();
-  double* tmp = c.eo_d[0];
-  deo<double>(c, tmp, in, c.pco, 3, 0, 1, 0, 0.0, nullptr);
-  deo<double>(c, out, tmp, c.pce, 3, 0, 1, 2, -c.kappa * c.kappa, in);
-  c.n_mtilde++;
+// (dee_deo_vm_(pco, pce) then one_minus_dee_deo_vm_(pce, pco)); compact, tmp
+// of the other parity
+static void mtilde_c(Ctx& c, double* out, const double* in, double* tmp) {
+  eo_apply<double>(c, tmp, in, c.pco, 3, 0, 1, 0, 0.0, nullptr);
+  eo_apply<double>(c, out, tmp, c.pce, 3, 0, 1, 2, -c.kappa * c.kappa, in);
+}
+// mtilde_dag_vm_: clvd_vm2_(pce), dee_deo_dag_vm_(pco, pce), one_minus_deo_dag_vm_(pce, pco)
+static void mtilde_dag_c(Ctx& c, double* out, const double* in, double* t0, double* t1) {
+  auto a = eo_args<double>(c, c.pce);
+  a.src = in;
+  a.out = t0;
+  launch_eo_clv<double>(a, c.st);
+  eo_apply<double>(c, t1, t0, c.pco, 3, 1, 1, 0, 0.0, nullptr);
+  eo_apply<double>(c, out, t1, c.pce, 3, 1, 0, 2, -c.kappa * c.kappa, in);
+}
+// mtdagmt_vm_: mtilde_dag(mtilde(in)); work: eo_d[0 .. 2]
+static void mtdagmt_c(Ctx& c, double* out, const double* in) {
+  mtilde_c(c, c.eo_d[2], in, c.eo_d[0]);
+  mtilde_dag_c(c, out, c.eo_d[2], c.eo_d[0], c.eo_d[1]);
 }
 
-// mtilde_dag_vm_: clvd_vm2_(pce), dee_deo_dag_vm_(pco, pce), one_minus_deo_dag_vm_(pce, pco)
+void mtilde_d(Ctx& c, double* out, const double* in) {
+  double** v = eo_vecs<double>(c, 3);
+  eo_gather<double>(c.G, v[1], c.eo_pad(), in, c.pce, c.st);
+  mtilde_c(c, v[2], v[1], v[0]);
+  eo_scatter<double>(c.G, out, v[2], c.eo_pad(), c.pce, 0, 0.0, nullptr, false, c.st);
+  c.n_mtilde++;
+  c.check_launch("mtilde_d");
+}
+
 void mtilde_dag_d(Ctx& c, double* out, const double* in) {
-  c.ensure_eo();
-  double *t0 = c.eo_d[0], *t1 = c.eo_d[1];
-  clv<double>(c, t0, in, c.pce);
-  deo<double>(c, t1, t0, c.pco, 3, 1, 1, 0, 0.0, nullptr);
-  deo<double>(c, out, t1, c.pce, 3, 1, 0, 2, -c.kappa * c.kappa, in);
+  double** v = eo_vecs<double>(c, 4);
+  eo_gather<double>(c.G, v[2], c.eo_pad(), in, c.pce, c.st);
+  mtilde_dag_c(c, v[3], v[2], v[0], v[1]);
+  eo_scatter<double>(c.G, out, v[3], c.eo_pad(), c.pce, 0, 0.0, nullptr, false, c.st);
+  c.check_launch("mtilde_dag_d");
 }
 
 void mtilde_s(Ctx& c, float* out, const float* in) {
-  c.ensure_eo();
-  float* tmp = c.eo_s[0];
-  deo<float>(c, tmp, in, c.pco, 3, 0, 1, 0, 0.0, nullptr);
-  deo<float>(c, out, tmp, c.pce, 3, 0, 1, 2, -(double)(float)(c.kappa * c.kappa), in);
+  float** v = eo_vecs<float>(c, 3);
+  eo_gather<float>(c.G, v[1], c.eo_pad(), in, c.pce, c.st);
+  eo_apply<float>(c, v[0], v[1], c.pco, 3, 0, 1, 0, 0.0, nullptr);
+  eo_apply<float>(c, v[2], v[0], c.pce, 3, 0, 1, 2, -(double)(float)(c.kappa * c.kappa), v[1]);
+  eo_scatter<float>(c.G, out, v[2], c.eo_pad(), c.pce, 0, 0.0f, nullptr, false, c.st);
+  c.check_launch("mtilde_s");
 }
 
 // bicgstab_vm_ (bicgstab.cc:68-333): BiCGStab on mtilde for the pce parity,
 // iter = 1..maxiter-1, converged when sqrt(|r|^2/|b|^2) < 1e-14 after the
 // omega step.  x: initial guess in, solution out.  Returns conviter.
 int bicgstab_vm(Ctx& c, double* x, const double* b, int maxiter) {
-  c.ensure_eo();
-  c.ensure_outer();
-  const Geom& G = c.G;
-  double *q = c.eo_d[2], *r = c.eo_d[3], *p = c.eo_d[4], *t = c.eo_d[5], *r0 = c.out_r0,
-         *bb = c.out_q, *xx = c.out_p;
-  // vectors of one parity: the other parity's sites are held at zero
-  parity_select<double>(G, bb, b, c.pce, c.st);
-  parity_select<double>(G, xx, x, c.pce, c.st);
-  mtilde_d(c, q, xx);
+  double** v = eo_vecs<double>(c, 8);
+  const Geom G = eo_geom(c);
+  double *tmp = v[0], *bb = v[1], *q = v[2], *r = v[3], *p = v[4], *t = v[5], *r0 = v[6],
+         *xx = v[7];
+  eo_gather<double>(c.G, bb, G.pad, b, c.pce, c.st);
+  eo_gather<double>(c.G, xx, G.pad, x, c.pce, c.st);
+  mtilde_c(c, q, xx, tmp);
   blas_bicg_init<double>(G, bb, q, r, p, r0, c.d_res, c.rb, c.st);
   const double* h = c.fetch(2);
   const double bnorm = h[0];
   std::complex<double> rho0(h[1], 0), rho, beta, omega, alpha, ctmp;
   int iter;
   for (iter = 1; iter < maxiter; iter++) {
-    mtilde_d(c, q, p);
+    mtilde_c(c, q, p, tmp);
     blas_cdot<double>(G, r0, q, c.d_res, c.rb, c.st);
     h = c.fetch(2);
     ctmp = std::complex<double>(h[0], h[1]);
     alpha = rho0 / ctmp;
     blas_bicg_update<double>(G, xx, r, p, q, alpha.real(), alpha.imag(), nullptr, c.d_res, c.rb,
                              c.st);
-    mtilde_d(c, t, r);
+    mtilde_c(c, t, r, tmp);
     blas_norm_cdot<double>(G, t, r, c.d_res, c.rb, c.st);
     h = c.fetch(3);
     omega = std::complex<double>(h[1] / h[0], h[2] / h[0]);
@@ -143,17 +245,17 @@ int bicgstab_vm(Ctx& c, double* x, const double* b, int maxiter) {
     rho0 = rho;
     blas_bicg_p<double>(G, p, r, q, beta.real(), beta.imag(), omega.real(), omega.imag(), c.st);
   }
-  blas_copy<double>(G, x, xx, 0, G.V, c.st);
+  eo_scatter<double>(c.G, x, xx, G.pad, c.pce, 0, 0.0, nullptr, true, c.st);
   c.check_launch("bicgstab_vm");
   return iter;
 }
 
-// mtdagmt_vm_: mtilde_dag(mtilde(in))
 void mtdagmt_d(Ctx& c, double* out, const double* in) {
-  c.ensure_eo();
-  double* t = c.eo_d[5];
-  mtilde_d(c, t, in);
-  mtilde_dag_d(c, out, t);
+  double** v = eo_vecs<double>(c, 4);
+  eo_gather<double>(c.G, v[3], c.eo_pad(), in, c.pce, c.st);
+  mtdagmt_c(c, v[3], v[3]);  // (in is last read before out is written)
+  eo_scatter<double>(c.G, out, v[3], c.eo_pad(), c.pce, 0, 0.0, nullptr, false, c.st);
+  c.check_launch("mtdagmt_d");
 }
 
 static void check_finite(double v, const char* what) {
@@ -166,25 +268,23 @@ static void check_finite(double v, const char* what) {
 // (the reference does not report it).  A zero source returns x = 0 at
 // iteration 0 (the reference divides 0 by 0 there).
 int cg_vm(Ctx& c, double* x, const double* b, int maxiter) {
-  c.ensure_eo();
-  c.ensure_outer();
-  const Geom& G = c.G;
-  double *q = c.eo_d[2], *r = c.eo_d[3], *p = c.eo_d[4], *r0 = c.out_r0, *bb = c.out_q,
-         *xx = c.out_p;
-  parity_select<double>(G, bb, b, c.pce, c.st);
-  parity_select<double>(G, xx, x, c.pce, c.st);
-  mtdagmt_d(c, q, xx);
+  double** v = eo_vecs<double>(c, 9);
+  const Geom G = eo_geom(c);
+  double *q = v[3], *r = v[4], *p = v[5], *r0 = v[6], *bb = v[7], *xx = v[8];
+  eo_gather<double>(c.G, bb, G.pad, b, c.pce, c.st);
+  eo_gather<double>(c.G, xx, G.pad, x, c.pce, c.st);
+  mtdagmt_c(c, q, xx);
   blas_bicg_init<double>(G, bb, q, r, p, r0, c.d_res, c.rb, c.st);
   const double* h = c.fetch(2);
   const double bnorm = h[0];
   double rho0 = h[1];
   if (bnorm == 0) {
-    blas_zero<double>(G, x, 0, G.V, c.st);
+    blas_zero<double>(c.G, x, 0, c.G.V, c.st);
     return 0;
   }
   int iter;
   for (iter = 1; iter < maxiter; iter++) {
-    mtdagmt_d(c, q, p);
+    mtdagmt_c(c, q, p);
     blas_cdot<double>(G, p, q, c.d_res, c.rb, c.st);
     h = c.fetch(1);
     const double alpha = rho0 / h[0];
@@ -197,7 +297,7 @@ int cg_vm(Ctx& c, double* x, const double* b, int maxiter) {
     rho0 = rnorm;
     blas_bicg_p<double>(G, p, r, q, beta, 0.0, 0.0, 0.0, c.st);
   }
-  blas_copy<double>(G, x, xx, 0, G.V, c.st);
+  eo_scatter<double>(c.G, x, xx, G.pad, c.pce, 0, 0.0, nullptr, true, c.st);
   c.check_launch("cg_vm");
   return iter;
 }
@@ -213,32 +313,37 @@ int cg_vm(Ctx& c, double* x, const double* b, int maxiter) {
 int mcg_vm(Ctx& c, double* X, const double* b, int n, const double* sigma, int maxiter) {
   if (n < 1 || n > Ctx::kMaxRhs) throw Error(1, "mcg_vm: number of shifts must be 1..32");
   if (c.G.nr != 1) throw Error(1, "mcg_vm: single right-hand side only");
-  c.ensure_eo();
-  c.ensure_outer();
-  const Geom& G = c.G;
+  double** v = eo_vecs<double>(c, 8);
+  const Geom G = eo_geom(c);
+  const size_t ne = (size_t)24 * G.pad;
   if (c.ms_n < n) {
-    c.ms_p = nullptr;
-    QWSG_CUDA(cudaMalloc(&c.ms_p, sizeof(double) * c.spinor_elems() * n));
-    c.owned.push_back(c.ms_p);
+    c.ms_p = c.ms_x = nullptr;  // (the smaller ones stay with the handle)
+    c.ms_n = 0;
+    eo_alloc(c, &c.ms_p, ne * n);
+    eo_alloc(c, &c.ms_x, ne * n);
     c.ms_n = n;
   }
-  double *q = c.eo_d[2], *r = c.eo_d[3], *p = c.eo_d[4], *r0 = c.out_r0, *bb = c.out_q;
-  parity_select<double>(G, bb, b, c.pce, c.st);
+  double *q = v[3], *r = v[4], *p = v[5], *r0 = v[6], *bb = v[7];
+  eo_gather<double>(c.G, bb, G.pad, b, c.pce, c.st);
   blas_bicg_init<double>(G, bb, nullptr, r, p, r0, c.d_res, c.rb, c.st);
   const double* h = c.fetch(1);
   const double bnorm = h[0];
   double rho0 = bnorm;
   for (int k = 0; k < n; k++) {
-    blas_zero<double>(G, X + k * c.spinor_elems(), 0, G.V, c.st);
-    blas_copy<double>(G, c.ms_p + k * c.spinor_elems(), r, 0, G.V, c.st);
+    blas_zero<double>(G, c.ms_x + k * ne, 0, G.V, c.st);
+    blas_copy<double>(G, c.ms_p + k * ne, r, 0, G.V, c.st);
   }
-  if (bnorm == 0) return 0;
+  if (bnorm == 0) {
+    for (int k = 0; k < n; k++)
+      blas_zero<double>(c.G, X + k * c.spinor_elems(), 0, c.G.V, c.st);
+    return 0;
+  }
   std::vector<double> z0(n, 1.0), z1(n, 1.0), z2(n, 0.0), cf(4 * n, 0.0);
   std::vector<char> active(n, 1);
   double alpha0 = 1.0, beta = 0.0;
   int iter;
   for (iter = 1; iter < maxiter; iter++) {
-    mtdagmt_d(c, q, p);
+    mtdagmt_c(c, q, p);
     blas_cdot<double>(G, p, q, c.d_res, c.rb, c.st);
     h = c.fetch(1);
     const double alpha = -rho0 / h[0];
@@ -258,7 +363,7 @@ int mcg_vm(Ctx& c, double* X, const double* b, int n, const double* sigma, int m
       cf[4 * k + 1] = z2[k];                   // pp_k = z2 r + ...
       cf[4 * k + 2] = beta_new * ratio * ratio;  // ... + beta (z2/z1)^2 pp_k
     }
-    blas_mshift(G, X, c.ms_p, n, r, p, beta_new, c.put_coefs(cf.data(), 4 * n), !done, c.st);
+    blas_mshift(G, c.ms_x, c.ms_p, n, r, p, beta_new, c.put_coefs(cf.data(), 4 * n), !done, c.st);
     if (done) break;
     beta = beta_new;
     rho0 = rnorm;
@@ -271,6 +376,9 @@ int mcg_vm(Ctx& c, double* X, const double* b, int n, const double* sigma, int m
     }
     alpha0 = alpha;
   }
+  for (int k = 0; k < n; k++)
+    eo_scatter<double>(c.G, X + k * c.spinor_elems(), c.ms_x + k * ne, G.pad, c.pce, 0, 0.0, nullptr,
+                       true, c.st);
   c.check_launch("mcg_vm");
   return iter;
 }

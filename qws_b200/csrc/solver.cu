@@ -293,7 +293,12 @@ void Ctx::ensure_hp() {
   }
   if (!h_isc) QWSG_CUDA(cudaMallocHost(&h_isc, sizeof(InnerScalars)));
 }
+long Ctx::next_fields_gen() {
+  static std::atomic<long> n{0};
+  return ++n;
+}
 void Ctx::ensure_fields_d() {
+  fields_gen_d = next_fields_gen();  // the compact even-odd copies follow the fields
   for (double** p : {&Ud, &Cd})
     if (!*p) {
       QWSG_CUDA(cudaMalloc(p, sizeof(double) * 72 * (size_t)G.pad));
@@ -301,6 +306,7 @@ void Ctx::ensure_fields_d() {
     }
 }
 void Ctx::ensure_fields_s() {
+  fields_gen_s = next_fields_gen();
   for (float** p : {&Us, &Cs})
     if (!*p) {
       QWSG_CUDA(cudaMalloc(p, sizeof(float) * 72 * (size_t)G.pad));
