@@ -220,7 +220,6 @@ inline int nb(long n) { return (int)((n + 127) / 128); }
 enum { CONV_S2H = 0, CONV_H2S = 1, CONV_H2H = 2 };
 template <int K>
 __device__ __forceinline__ void conv_entry(const Geom& G, void* dst, const void* src, int e) {
-  if (e >= (G.V << G.lgnr)) return;
   const int sp = spad(G);
   if (K == CONV_S2H) {
     float v[24];
@@ -241,13 +240,16 @@ __device__ __forceinline__ void conv_entry(const Geom& G, void* dst, const void*
   }
 }
 __global__ void k_s2h(Geom G, __half* dst, const float* __restrict__ src) {
-  conv_entry<CONV_S2H>(G, dst, src, blockIdx.x * blockDim.x + threadIdx.x);
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < G.V) conv_entry<CONV_S2H>(G, dst, src, e);
 }
 __global__ void k_h2s(Geom G, float* dst, const __half* __restrict__ src) {
-  conv_entry<CONV_H2S>(G, dst, src, blockIdx.x * blockDim.x + threadIdx.x);
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < G.V) conv_entry<CONV_H2S>(G, dst, src, e);
 }
-__global__ void k_h2h(Geom G, __half* dst, const __half* __restrict__ src) {
-  conv_entry<CONV_H2H>(G, dst, src, blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void k_h2h(Geom G, __half* dst, const __half* __restrict__ src, int e0, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) conv_entry<CONV_H2H>(G, dst, src, e0 + i);
 }
 
 // the same conversions for several lattices in one launch (group solves;
@@ -256,6 +258,7 @@ struct ConvArgs {
   Geom G;
   void* dst;
   const void* src;
+  int e0, n;  // entries [e0, e0 + n)
 };
 template <int K>
 __global__ void k_conv_multi(const ConvArgs* __restrict__ args, const int* __restrict__ starts,
@@ -263,7 +266,8 @@ __global__ void k_conv_multi(const ConvArgs* __restrict__ args, const int* __res
   __shared__ ConvArgs sa;
   const int l = group_member(starts, n, blockIdx.x);
   group_load_args(sa, args + l);
-  conv_entry<K>(sa.G, sa.dst, sa.src, (blockIdx.x - starts[l]) * blockDim.x + threadIdx.x);
+  const int i = (blockIdx.x - starts[l]) * blockDim.x + threadIdx.x;
+  if (i < sa.n) conv_entry<K>(sa.G, sa.dst, sa.src, sa.e0 + i);
 }
 template <int K>
 void merge_conv(const GroupRec* const* recs, int n, GroupBatch& b) {
@@ -273,9 +277,10 @@ void merge_conv(const GroupRec* const* recs, int n, GroupBatch& b) {
   for (int l = 0; l < n; l++) {
     args[l] = group_arg<ConvArgs>(recs[l]);
     starts[l] = blocks;
-    blocks += (args[l].G.V + 127) / 128;
+    blocks += (args[l].n + 127) / 128;
   }
   starts[n] = blocks;
+  if (blocks == 0) return;
   const size_t oa = b.put(args.data(), sizeof(ConvArgs) * n), os = b.put_starts(starts);
   b.launches.push_back([=](const unsigned char* dev, cudaStream_t st) {
     count_launch();
@@ -284,10 +289,10 @@ void merge_conv(const GroupRec* const* recs, int n, GroupBatch& b) {
   });
 }
 template <int K>
-bool record_conv(const Geom& G, void* dst, const void* src) {
+bool record_conv(const Geom& G, void* dst, const void* src, int site0, int n) {
   if (!g_group_rec) return false;
   if (G.nr != 1) group_unrecorded_launch();
-  return group_record(&merge_conv<K>, ConvArgs{G, dst, src});
+  return group_record(&merge_conv<K>, ConvArgs{G, dst, src, site0, n});
 }
 
 // the same three conversions for FP16 fields of two or more RHS (IOP
@@ -319,9 +324,9 @@ __global__ void k_h2s_pair(Geom G, float* dst, const __half* __restrict__ src) {
   IO<float>::store_spinor(dst, sp, 2 * e, a);
   IO<float>::store_spinor(dst, sp, 2 * e + 1, b);
 }
-__global__ void k_h2h_pair(Geom G, __half* dst, const __half* __restrict__ src) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (G.V << (G.lgnr - 1))) return;
+__global__ void k_h2h_pair(Geom G, __half* dst, const __half* __restrict__ src, int e0, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, e = e0 + i;
+  if (i >= n) return;
   const size_t pp = spad(G) >> 1;
   const uint4* s = reinterpret_cast<const uint4*>(src);
   uint4* d = reinterpret_cast<uint4*>(dst);
@@ -419,7 +424,7 @@ void links_compress12(const Geom& G, float* U12, const float* Us, cudaStream_t s
 // FP16 spinors of one RHS use IO<H16>, of two or more the IOP layout of the
 // paired hop kernels
 void spinor_s2h(const Geom& G, __half* dst, const float* src, cudaStream_t st) {
-  if (record_conv<CONV_S2H>(G, dst, src)) return;
+  if (record_conv<CONV_S2H>(G, dst, src, 0, G.V)) return;
   count_launch();
   if (G.nr >= 2)
     k_s2h_pair<<<nb(G.V << (G.lgnr - 1)), 128, 0, st>>>(G, dst, src);
@@ -427,20 +432,23 @@ void spinor_s2h(const Geom& G, __half* dst, const float* src, cudaStream_t st) {
     k_s2h<<<nb(G.V), 128, 0, st>>>(G, dst, src);
 }
 void spinor_h2s(const Geom& G, float* dst, const __half* src, cudaStream_t st) {
-  if (record_conv<CONV_H2S>(G, dst, src)) return;
+  if (record_conv<CONV_H2S>(G, dst, src, 0, G.V)) return;
   count_launch();
   if (G.nr >= 2)
     k_h2s_pair<<<nb(G.V << (G.lgnr - 1)), 128, 0, st>>>(G, dst, src);
   else
     k_h2s<<<nb(G.V), 128, 0, st>>>(G, dst, src);
 }
-void spinor_h2h(const Geom& G, __half* dst, const __half* src, cudaStream_t st) {
-  if (record_conv<CONV_H2H>(G, dst, src)) return;
+void spinor_h2h(const Geom& G, __half* dst, const __half* src, int site0, int n, cudaStream_t st) {
+  if (n <= 0) return;
+  if (record_conv<CONV_H2H>(G, dst, src, site0, n)) return;
   count_launch();
-  if (G.nr >= 2)
-    k_h2h_pair<<<nb(G.V << (G.lgnr - 1)), 128, 0, st>>>(G, dst, src);
-  else
-    k_h2h<<<nb(G.V), 128, 0, st>>>(G, dst, src);
+  if (G.nr >= 2) {
+    const int lg = G.lgnr - 1;
+    k_h2h_pair<<<nb((long)n << lg), 128, 0, st>>>(G, dst, src, site0 << lg, n << lg);
+  } else {
+    k_h2h<<<nb(n), 128, 0, st>>>(G, dst, src, site0, n);
+  }
 }
 void fields_s2h(const Geom& G, __half* Uh, const float* Us, __half* Ch, const float* Cs,
                 cudaStream_t st) {

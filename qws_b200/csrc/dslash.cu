@@ -13,7 +13,8 @@
 //                 x <- b + kappa A^-1 H_blk x, algebraically the reference's
 //                 x + (b - D_blk x), static_solver.cc:77-139)
 //        EPI_SAPE out = out + (aux - (src - kappa*acc)) (s_e += in_e - D_blk a_e,
-//                 qws.cc:815-818 with the ddd_in result kept in registers)
+//                 qws.cc:815-818 with the ddd_in result kept in registers; with
+//                 all hops also s_e += kappa A^-1 H_face a, see sap_t)
 //   T    storage format (float, double, H16); arithmetic in Arith<T>::R.
 // Faces are not packed: a face hop reads the neighbouring block's site of
 // the source field directly from HBM (the whole lattice is resident).
@@ -220,7 +221,7 @@ __device__ __forceinline__ void hop_site_at(const HopArgs<T>& a, const int i) {
     for (int j = 0; j < 24; j++) o[j] = madd(coef, acc[j], o[j]);
   } else {  // EPI_SAPE: coef = -kappa
     V in[24], av[24];
-    P::load(a.out, pd, e, o);
+    P::load(a.sin ? a.sin : a.out, pd, e, o);
     P::load(a.aux, pd, e, in);
     P::load(a.src, pd, e, av);
 #pragma unroll
@@ -306,7 +307,7 @@ static void launch_v(const HopArgs<T>& a, cudaStream_t st) {
     return;
   }
   if constexpr (!PRK && ((SEL == HOP_ALL && std::is_same<T, float>::value) ||
-                         (SEL == HOP_OUTER && std::is_same<T, H16>::value))) {
+                         (SEL != HOP_INNER && std::is_same<T, H16>::value))) {
     if (threads == 128) {  // (the bound assumes CTAs of at most 128 threads)
       k_hop_r73<T, SEL, EPI, PRK><<<blocks, threads, 0, st>>>(a);
       return;
@@ -372,6 +373,9 @@ void launch_hop(int sel, int epi, const HopArgs<T>& a, cudaStream_t st) {
     QWSG_CASE(HOP_OUTER, EPI_ADD)
     QWSG_CASE(HOP_INNER, EPI_JINV)
     QWSG_CASE(HOP_INNER, EPI_SAPE)
+    if constexpr (!std::is_same<T, double>::value) {
+      QWSG_CASE(HOP_ALL, EPI_SAPE)
+    }
 #undef QWSG_CASE
   }
 #define QWSG_CASE(S, E)              \
@@ -384,6 +388,9 @@ void launch_hop(int sel, int epi, const HopArgs<T>& a, cudaStream_t st) {
   QWSG_CASE(HOP_OUTER, EPI_ADD)
   QWSG_CASE(HOP_INNER, EPI_JINV)
   QWSG_CASE(HOP_INNER, EPI_SAPE)
+  if constexpr (!std::is_same<T, double>::value) {
+    QWSG_CASE(HOP_ALL, EPI_SAPE)
+  }
 #undef QWSG_CASE
 }
 

@@ -101,6 +101,8 @@ __device__ __forceinline__ void group_load_args(A& dst, const A* __restrict__ sr
 #endif
 
 enum { HOP_INNER = 1, HOP_OUTER = 2, HOP_ALL = 3 };
+// EPI_SAPE goes with HOP_INNER (the SAP update alone) and HOP_ALL (the update
+// and the face hops onto the same sites in one pass)
 enum { EPI_D = 0, EPI_ADD = 1, EPI_JINV = 2, EPI_SAPE = 3 };
 
 // T: storage tag (float, double, H16 = FP16 storage / FP32 arithmetic)
@@ -110,6 +112,7 @@ struct HopArgs {
   Geom G;
   const S* src;   // field the hops read
   const S* aux;   // b (EPI_JINV) or the SAP right-hand side `in` (EPI_SAPE)
+  const S* sin;   // EPI_SAPE: the s to update (null: out, in place)
   S* out;
   const S* U;     // gauge planes
   const S* U12;   // FP32 only: links in 12-real form (null: use U)
@@ -238,7 +241,8 @@ void links_compress12(const Geom& G, float* U12, const float* Us, cudaStream_t s
 // FP32 planes <-> FP16 planes with per-site scales (IO<H16> format)
 void spinor_s2h(const Geom& G, __half* dst, const float* src, cudaStream_t st);
 void spinor_h2s(const Geom& G, float* dst, const __half* src, cudaStream_t st);
-void spinor_h2h(const Geom& G, __half* dst, const __half* src, cudaStream_t st);
+// sites [site0, site0 + n)
+void spinor_h2h(const Geom& G, __half* dst, const __half* src, int site0, int n, cudaStream_t st);
 // FP16 copies of the FP32 gauge (9 complex planes per mu) and clover planes
 void fields_s2h(const Geom& G, __half* Uh, const float* Us, __half* Ch, const float* Cs,
                 cudaStream_t st);
