@@ -267,6 +267,307 @@ __global__ void __launch_bounds__(256) k_hop_pair(const HopArgs<H16> a) {
   hop_site<H16, TwoRhs, SEL, EPI, PRK>(a);
 }
 
+// ---------------------------------------------------------------------------
+// Four threads per site (one RHS; FP32 and FP16): a CTA of four warps handles
+// 32 sites.  Warp w first computes the two hops along direction w (projection
+// and link product), then owns spin w: it adds the eight hops' contributions
+// to that spin, makes three rows of A^-1 x and writes the spin's six reals.
+// What the warps exchange goes through shared memory.  Every sum runs in the
+// order of hop_site_at, so the results are bit for bit the same.
+//
+// For launches that leave the chip underfilled, where the time is one thread's
+// chain of loads and its ~1,900 instructions: a quarter of the chain per
+// thread and four times the warps.
+// ---------------------------------------------------------------------------
+// Most sites of such a launch.  Measured per SAP application (one thread ->
+// four threads a site): FP32 at 2,048 sites a launch 188 -> 98 us, 20,736:
+// 224 -> 173, 27,440: 242 -> 213, 38,416: 265 -> 281; FP16 (more instructions
+// a site, so an SM fills earlier) 150 -> 102, 190 -> 172, 198 -> 207,
+// 222 -> 268.
+template <typename T>
+constexpr int kSplitSites = std::is_same<T, H16>::value ? 148 * 144 : 148 * 192;
+struct SplitShared {
+  float2 r[8][6][32];   // hop 2 mu + (dir < 0): link product, [2 colour + k]
+  float f[8][32];       // and its factor (0: the hop does not count)
+  float2 x[4][3][32];   // summed spins, [spin][colour]
+  float2 y[2][6][32];   // A^-1 x of the two chiral blocks
+  float m[4][32];       // FP16 storage: largest component of each spin
+};
+
+// link product of one hop into shared memory
+template <typename T, int SEL, int MU, int DIR>
+__device__ __forceinline__ void split_hop(const HopArgs<T>& a, const Site& s, int g, bool live,
+                                          int lane, SplitShared& sh) {
+  constexpr int k = 2 * MU + (DIR < 0);
+  const bool face = DIR > 0 ? (s.lc[MU] == a.G.B[MU] - 1) : (s.lc[MU] == 0);
+  bool on = live && (face ? (SEL & HOP_OUTER) != 0 : (SEL & HOP_INNER) != 0);
+  int gn = g;
+  if (on) {
+    if (!face) {
+      gn = g + rot_step(a.G, MU, s.lc[MU], DIR);
+    } else {
+      int ncol;
+      gn = nbr_across(a.G, s, MU, DIR, &ncol);
+      on = ncol != a.zero_col;
+    }
+  }
+  float r[12], f = 0;
+  if (on) {
+    float v[24], sc, h[12], u[18];
+    if (MU == 3)
+      IO<T>::load_half_raw(a.src, a.G.pad, gn, DIR > 0, v, sc);
+    else
+      IO<T>::load_spinor_raw(a.src, a.G.pad, gn, v, sc);
+    if constexpr (std::is_same<T, float>::value) {
+      if (a.U12)
+        load_link12(a.U12, a.G.pad, MU, DIR > 0 ? g : gn, u);
+      else
+        IO<T>::load_link(a.U, a.G.pad, MU, DIR > 0 ? g : gn, u);
+    } else {
+      IO<T>::load_link(a.U, a.G.pad, MU, DIR > 0 ? g : gn, u);
+    }
+    project<float, MU, DIR>(v, h);
+    if (DIR > 0)
+      link_mul<float, false>(u, h, r);
+    else
+      link_mul<float, true>(u, h, r);
+    f = sc;
+    if (MU == 3) {
+      f = 2.0f * sc;
+      if (face && (DIR > 0 ? s.bc[3] == a.G.NB[3] - 1 : s.bc[3] == 0))
+        f = (float)(2 * a.G.tbc) * sc;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 12; j++) r[j] = 0;
+  }
+#pragma unroll
+  for (int j = 0; j < 6; j++) sh.r[k][j][lane] = make_float2(r[2 * j], r[2 * j + 1]);
+  sh.f[k][lane] = f;
+}
+
+// the contribution of hop (MU, DIR) to spin SPIN (the rows of reconstruct)
+template <int SPIN, int MU, int DIR>
+__device__ __forceinline__ void split_add(const SplitShared& sh, int lane, float acc[6]) {
+  if (MU == 3 && (DIR > 0 ? SPIN < 2 : SPIN >= 2)) return;
+  constexpr int hop = 2 * MU + (DIR < 0);
+  // which of the two projected spins, and as it is (+-1) or times +-i
+  constexpr int k = SPIN < 2 || MU == 3 ? SPIN & 1 : MU == 2 ? SPIN - 2 : 3 - SPIN;
+  constexpr bool times_i = SPIN >= 2 && (MU == 0 || MU == 2);
+  constexpr int up = DIR > 0 ? 1 : -1;
+  constexpr int sgn = SPIN < 2 || MU == 3 ? 1
+                      : MU == 0           ? up
+                      : MU == 1           ? (SPIN == 2 ? up : -up)
+                                          : (SPIN == 2 ? up : -up);
+  const float f = sh.f[hop][lane], p = sgn > 0 ? f : -f;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const float2 r = sh.r[hop][2 * c + k][lane];
+    if (times_i) {
+      acc[2 * c] = madd(-p, r.y, acc[2 * c]);
+      acc[2 * c + 1] = madd(p, r.x, acc[2 * c + 1]);
+    } else {
+      acc[2 * c] = madd(p, r.x, acc[2 * c]);
+      acc[2 * c + 1] = madd(p, r.y, acc[2 * c + 1]);
+    }
+  }
+}
+template <int SPIN>
+__device__ __forceinline__ void split_sum(const SplitShared& sh, int lane, float acc[6]) {
+#pragma unroll
+  for (int j = 0; j < 6; j++) acc[j] = 0;
+  split_add<SPIN, 0, +1>(sh, lane, acc);
+  split_add<SPIN, 0, -1>(sh, lane, acc);
+  split_add<SPIN, 1, +1>(sh, lane, acc);
+  split_add<SPIN, 1, -1>(sh, lane, acc);
+  split_add<SPIN, 2, +1>(sh, lane, acc);
+  split_add<SPIN, 2, -1>(sh, lane, acc);
+  split_add<SPIN, 3, +1>(sh, lane, acc);
+  split_add<SPIN, 3, -1>(sh, lane, acc);
+}
+
+// rows 3 H .. 3 H + 2 of A x, A the Hermitian block a (clover_apply_with's
+// order: for row j the columns 0 .. 5 but j, after the diagonal)
+template <int H>
+__device__ __forceinline__ void split_clover(const float a[36], const float2 x[6], float2 y[3]) {
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    constexpr int kFirst = 3 * H;
+    const int j = kFirst + q;
+    float yr = a[j] * x[j].x, yi = a[j] * x[j].y;
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      if (k == j) continue;
+      const int lo = k < j ? k : j, hi = k < j ? j : k;
+      const int n = lo * 5 - lo * (lo - 1) / 2 + (hi - lo - 1);  // pair (lo, hi)
+      const float mr = a[6 + 2 * n], mi = a[7 + 2 * n], nmi = -a[7 + 2 * n];
+      yr = madd(mr, x[k].x, yr);
+      yr = madd(k < j ? mi : nmi, x[k].y, yr);
+      yi = madd(mr, x[k].y, yi);
+      yi = madd(k < j ? nmi : mi, x[k].x, yi);
+    }
+    y[q] = make_float2(yr, yi);
+  }
+}
+
+// the six reals of one spin of an FP32 or FP16 spinor, as stored, and the
+// site's scale
+template <typename T>
+struct SpinIO;
+template <>
+struct SpinIO<float> {
+  __device__ __forceinline__ static void load(const float* p, int pad, int g, int spin, float v[6],
+                                              float& s) {
+    s = 1.0f;
+    const float2* q = reinterpret_cast<const float2*>(p);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const float2 t = __ldg(q + 2 * ((size_t)(2 * c + (spin >> 1)) * pad + g) + (spin & 1));
+      v[2 * c] = t.x;
+      v[2 * c + 1] = t.y;
+    }
+  }
+};
+template <>
+struct SpinIO<H16> {
+  // 4-byte word of (colour, spin) of site g in the IO<H16> planes
+  __device__ __forceinline__ static size_t word(int pad, int g, int spin, int c) {
+    return c < 2 ? 4 * ((size_t)(spin >> 1) * pad + g) + 2 * c + (spin & 1)
+                 : 4 * ((size_t)2 * pad + g) + spin;
+  }
+  __device__ __forceinline__ static void load(const __half* p, int pad, int g, int spin, float v[6],
+                                              float& s) {
+    s = IO<H16>::scale(p, pad, g);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const unsigned w = __ldg(reinterpret_cast<const unsigned*>(p) + word(pad, g, spin, c));
+      __half2 h;
+      memcpy(&h, &w, 4);
+      const float2 t = __half22float2(h);
+      v[2 * c] = t.x;
+      v[2 * c + 1] = t.y;
+    }
+  }
+};
+
+template <typename T, int SEL, int EPI>
+__global__ void __launch_bounds__(128) k_hop_split(const HopArgs<T> a) {
+  __shared__ SplitShared sh;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  bool live = i < a.nsites;
+  const int ii = live ? i : a.nsites - 1;  // (a valid site for the idle lanes)
+  const int g = a.list ? __ldg(a.list + ii) : a.site0 + ii;
+  const int pad = a.G.pad;
+  Site s;
+  decode_site(a.G, g, s);
+  if (a.dom >= 0 && (s.bc[0] & 1) != a.dom) live = false;
+  if (SEL == HOP_OUTER) {
+    bool face = false;
+#pragma unroll
+    for (int mu = 0; mu < 4; mu++) face |= (s.lc[mu] == 0) | (s.lc[mu] == a.G.B[mu] - 1);
+    live = live && face;
+  }
+  switch (w) {
+    case 0:
+      split_hop<T, SEL, 0, +1>(a, s, g, live, lane, sh);
+      split_hop<T, SEL, 0, -1>(a, s, g, live, lane, sh);
+      break;
+    case 1:
+      split_hop<T, SEL, 1, +1>(a, s, g, live, lane, sh);
+      split_hop<T, SEL, 1, -1>(a, s, g, live, lane, sh);
+      break;
+    case 2:
+      split_hop<T, SEL, 2, +1>(a, s, g, live, lane, sh);
+      split_hop<T, SEL, 2, -1>(a, s, g, live, lane, sh);
+      break;
+    default:
+      split_hop<T, SEL, 3, +1>(a, s, g, live, lane, sh);
+      split_hop<T, SEL, 3, -1>(a, s, g, live, lane, sh);
+  }
+  // this warp's chiral block and the epilogue's operands, while the others hop
+  const int blk = w >> 1;
+  float cl[36], o[6], in[6], av[6], so, si, sa;
+  if (blk == 0)
+    IO<T>::load_clover_block(a.C, pad, g, 0, cl);
+  else
+    IO<T>::load_clover_block(a.C, pad, g, 1, cl);
+  SpinIO<T>::load(EPI == EPI_D ? a.src : EPI == EPI_JINV ? a.aux : EPI == EPI_SAPE && a.sin ? a.sin
+                                                                                        : a.out,
+                  pad, g, w, o, so);
+  if (EPI == EPI_SAPE) {
+    SpinIO<T>::load(a.aux, pad, g, w, in, si);
+    SpinIO<T>::load(a.src, pad, g, w, av, sa);
+  }
+  __syncthreads();
+  float acc[6];
+  switch (w) {
+    case 0: split_sum<0>(sh, lane, acc); break;
+    case 1: split_sum<1>(sh, lane, acc); break;
+    case 2: split_sum<2>(sh, lane, acc); break;
+    default: split_sum<3>(sh, lane, acc);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++) sh.x[w][c][lane] = make_float2(acc[2 * c], acc[2 * c + 1]);
+  __syncthreads();
+  float2 x[6], y[3];
+#pragma unroll
+  for (int j = 0; j < 6; j++) {  // rows 0-2: s0 +- s2, rows 3-5: s1 +- s3
+    const float2 p = sh.x[j / 3][j % 3][lane], q = sh.x[2 + j / 3][j % 3][lane];
+    x[j] = blk == 0 ? make_float2(p.x + q.x, p.y + q.y) : make_float2(p.x - q.x, p.y - q.y);
+  }
+  if ((w & 1) == 0)
+    split_clover<0>(cl, x, y);
+  else
+    split_clover<1>(cl, x, y);
+#pragma unroll
+  for (int c = 0; c < 3; c++) sh.y[blk][3 * (w & 1) + c][lane] = y[c];
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const float2 p = sh.y[1 - blk][3 * (w & 1) + c][lane];
+    acc[2 * c] = blk == 0 ? y[c].x + p.x : p.x - y[c].x;
+    acc[2 * c + 1] = blk == 0 ? y[c].y + p.y : p.y - y[c].y;
+  }
+#pragma unroll
+  for (int j = 0; j < 6; j++) {
+    if (EPI == EPI_SAPE) {  // (the roundings hop_site_at's expression comes out with)
+      const float m = madd(a.coef, acc[j], __fmul_rn(av[j], sa));
+      o[j] = __fmaf_rn(o[j], so, __fmaf_rn(in[j], si, -m));
+    } else {
+      o[j] = madd(a.coef, acc[j], __fmul_rn(o[j], so));
+    }
+  }
+  if constexpr (std::is_same<T, float>::value) {
+    if (!live) return;
+    float2* q = reinterpret_cast<float2*>(a.out);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+      q[2 * ((size_t)(2 * c + blk) * pad + g) + (w & 1)] = make_float2(o[2 * c], o[2 * c + 1]);
+  } else {  // IO<H16>::store_spinor
+    float n = 0;
+#pragma unroll
+    for (int j = 0; j < 6; j++) n = fmaxf(n, fabsf(o[j]));
+    sh.m[w][lane] = n;
+    __syncthreads();
+    if (!live) return;
+#pragma unroll
+    for (int k = 0; k < 4; k++) n = fmaxf(n, sh.m[k][lane]);
+    const bool keep = n >= 1e-30f;
+    const float inv = keep ? 1.0f / n : 0.0f;
+    unsigned* q = reinterpret_cast<unsigned*>(a.out);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const __half2 h = __floats2half2_rn(o[2 * c] * inv, o[2 * c + 1] * inv);
+      unsigned t;
+      memcpy(&t, &h, 4);
+      q[SpinIO<H16>::word(pad, g, w, c)] = t;
+    }
+    if (w == 0)
+      reinterpret_cast<float*>(reinterpret_cast<uint4*>(a.out) + (size_t)3 * pad)[g] = keep ? n : 0.0f;
+  }
+}
+
 // Several lattices in one launch (a group solve; one right-hand side each):
 // block b runs threads [(b - starts[l]) * blockDim, ...) of member l's own
 // launch, with l's arguments copied into shared memory first, so every
@@ -298,6 +599,12 @@ static void launch_v(const HopArgs<T>& a, cudaStream_t st) {
     if (a.G.nr >= 2) {
       const int blocks = ((a.nsites << (a.G.lgnr - 1)) + threads - 1) / threads;
       k_hop_pair<SEL, EPI, PRK><<<blocks, threads, 0, st>>>(a);
+      return;
+    }
+  }
+  if constexpr (!PRK && !std::is_same<T, double>::value) {
+    if (a.G.nr == 1 && a.nsites <= kSplitSites<T>) {
+      k_hop_split<T, SEL, EPI><<<(a.nsites + 31) / 32, 128, 0, st>>>(a);
       return;
     }
   }
