@@ -281,11 +281,12 @@ __global__ void __launch_bounds__(256) k_hop_pair(const HopArgs<H16> a) {
 // ---------------------------------------------------------------------------
 // Most sites of such a launch.  Measured per SAP application (one thread ->
 // four threads a site): FP32 at 2,048 sites a launch 188 -> 98 us, 20,736:
-// 224 -> 173, 27,440: 242 -> 213, 38,416: 265 -> 281; FP16 (more instructions
+// 224 -> 173, 27,440: 242 -> 213, 38,416: 265 -> 281 (D alone at 30,240 sites
+// 10.2 -> 8.2, at 38,416 10.4 -> 12.2); FP16 (more instructions
 // a site, so an SM fills earlier) 150 -> 102, 190 -> 172, 198 -> 207,
 // 222 -> 268.
 template <typename T>
-constexpr int kSplitSites = std::is_same<T, H16>::value ? 148 * 144 : 148 * 192;
+constexpr int kSplitSites = std::is_same<T, H16>::value ? 148 * 144 : 148 * 216;
 struct SplitShared {
   float2 r[8][6][32];   // hop 2 mu + (dir < 0): link product, [2 colour + k]
   float f[8][32];       // and its factor (0: the hop does not count)

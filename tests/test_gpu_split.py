@@ -2,7 +2,7 @@
 kernels, which a handle with two right-hand sides runs: FP32 results equal bit
 for bit, on site counts that leave the last CTA of 32 sites partly filled,
 with 12-real and full links, and on both sides of the size at which launches
-change over (FP16 21,312 and FP32 28,416 sites a launch)."""
+change over (FP16 21,312 and FP32 31,968 sites a launch)."""
 import numpy as np
 import pytest
 
