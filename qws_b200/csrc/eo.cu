@@ -34,6 +34,18 @@ __device__ __forceinline__ int eo_index(const Geom& G, const int x[4]) {
   return (x[0] >> 1) + (G.L[0] >> 1) * (x[1] + G.L[1] * (x[2] + G.L[2] * x[3]));
 }
 
+// coordinates of entry e of parity p
+__device__ __forceinline__ void eo_coords(const Geom& G, int e, int p, int x[4]) {
+  const int nxh = G.L[0] >> 1;
+  int k = e / nxh;
+  const int xh = e - k * nxh;
+  x[1] = k % G.L[1];
+  k /= G.L[1];
+  x[3] = k / G.L[2];
+  x[2] = k - x[3] * G.L[2];
+  x[0] = 2 * xh + ((p + x[1] + x[2] + x[3]) & 1);
+}
+
 struct EoSite {
   int xh, y, z, t;
   int odd;  // x = 2 xh + odd
@@ -157,20 +169,20 @@ __global__ void __launch_bounds__(128) k_clv(Geom G, T* out, const T* __restrict
   IO<T>::store_spinor(out, G.pad, g, v);
 }
 
-// full planes -> compact vector of parity pe.  Walked in the planes' order:
-// reads are runs, each write is a sector that its neighbour's write completes
-// in L2.
+// Conversions walk the order of what they write: a scattered 16-byte read costs
+// a sector, a scattered write a partly written one (FP64 at 24^3x48: gather
+// 38 us so, 69 in the planes' order; scatter 57, 129 in compact order).
+// full planes -> compact vector of parity pe
 template <typename T>
 __global__ void __launch_bounds__(128) k_eo_gather(Geom G, T* __restrict__ dst, int pad,
                                                    const T* __restrict__ src, int pe) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= G.V) return;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= G.Vh) return;
   int x[4];
-  site_coords(G, g, x);
-  if (((x[0] + x[1] + x[2] + x[3]) & 1) != pe) return;
+  eo_coords(G, e, pe, x);
   T v[24];
-  IO<T>::load_spinor(src, G.pad, g, v);
-  IO<T>::store_spinor(dst, pad, eo_index(G, x), v);
+  IO<T>::load_spinor(src, G.pad, dd_index(G, x), v);
+  IO<T>::store_spinor(dst, pad, e, v);
 }
 // compact vector -> parity pe of full planes: MODE 0 out = v, 1 out += coef v,
 // 2 out = in0 + coef v; ZERO: the other parity becomes zero (else untouched)
@@ -206,11 +218,11 @@ __global__ void __launch_bounds__(128) k_eo_scatter(Geom G, T* out, const T* __r
 template <typename T>
 __global__ void __launch_bounds__(128) k_eo_links(Geom G, T* __restrict__ dst, int pad,
                                                   const T* __restrict__ U) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= G.V) return;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, p = blockIdx.z;
+  if (e >= G.Vh) return;
   int x[4];
-  site_coords(G, g, x);
-  const int p = (x[0] + x[1] + x[2] + x[3]) & 1, e = eo_index(G, x);
+  eo_coords(G, e, p, x);
+  const int g = dd_index(G, x);
   T u[18];
   IO<T>::load_link(U, G.pad, blockIdx.y, g, u);
   store_link<T>(dst + (size_t)72 * pad * p, pad, blockIdx.y, e, u);
@@ -218,29 +230,31 @@ __global__ void __launch_bounds__(128) k_eo_links(Geom G, T* __restrict__ dst, i
 template <typename T>
 __global__ void __launch_bounds__(128) k_eo_clover(Geom G, T* __restrict__ dst, int pad,
                                                    const T* __restrict__ C) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= G.V) return;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, p = blockIdx.z;
+  if (e >= G.Vh) return;
   int x[4];
-  site_coords(G, g, x);
-  const int p = (x[0] + x[1] + x[2] + x[3]) & 1, e = eo_index(G, x);
-  T a[72];
-  IO<T>::load_clover_block(C, G.pad, g, 0, a);
-  IO<T>::load_clover_block(C, G.pad, g, 1, a + 36);
-  store_clover<T>(dst + (size_t)72 * pad * p, pad, e, a);
+  eo_coords(G, e, p, x);
+  const int g = dd_index(G, x);
+  // one chiral block's 16-byte planes
+  constexpr int n = 36 * sizeof(T) / 16;
+  const uint4* s = reinterpret_cast<const uint4*>(C) + (size_t)n * blockIdx.y * G.pad + g;
+  uint4* d = reinterpret_cast<uint4*>(dst + (size_t)72 * pad * p) + (size_t)n * blockIdx.y * pad + e;
+#pragma unroll
+  for (int j = 0; j < n; j++) d[(size_t)j * pad] = __ldg(s + (size_t)j * G.pad);
 }
 
 template <typename T>
 void eo_fields(const Geom& G, T* Ue, T* Ce, int pad, const T* U, const T* C, cudaStream_t st) {
-  const int nb = (G.V + 127) / 128;
+  const int nb = (G.Vh + 127) / 128;
   count_launch();
-  k_eo_links<T><<<dim3(nb, 4), 128, 0, st>>>(G, Ue, pad, U);
+  k_eo_links<T><<<dim3(nb, 4, 2), 128, 0, st>>>(G, Ue, pad, U);
   count_launch();
-  k_eo_clover<T><<<nb, 128, 0, st>>>(G, Ce, pad, C);
+  k_eo_clover<T><<<dim3(nb, 2, 2), 128, 0, st>>>(G, Ce, pad, C);
 }
 template <typename T>
 void eo_gather(const Geom& G, T* dst, int pad, const T* src, int pe, cudaStream_t st) {
   count_launch();
-  k_eo_gather<T><<<(G.V + 127) / 128, 128, 0, st>>>(G, dst, pad, src, pe);
+  k_eo_gather<T><<<(G.Vh + 127) / 128, 128, 0, st>>>(G, dst, pad, src, pe);
 }
 template <typename T>
 void eo_scatter(const Geom& G, T* out, const T* v, int pad, int pe, int mode, T coef, const T* in0,
