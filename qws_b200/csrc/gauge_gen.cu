@@ -228,14 +228,17 @@ double gen_gauge_device(Ctx& c, unsigned long long seed, int n_smear, double alp
   count_launch();
   k_d2f_planes<<<(unsigned)((n + 255) / 256), 256, 0, c.st>>>(c.Ud, c.Us, n);
   const int pb = (G.V + 127) / 128;
-  double* part = nullptr;  // stream-ordered: no device-wide synchronisation
-  QWSG_CUDA(cudaMallocAsync(&part, sizeof(double) * pb, c.st));
+  // the handle's reduction partials hold a sum per block of up to 19 million
+  // sites (an allocation here, stream-ordered, took 2 to 10 ms of the call)
+  const bool fits = (size_t)pb <= (size_t)4 * Ctx::kMaxRhs * c.rb.nblk;
+  double* part = c.rb.partial;
+  if (!fits) QWSG_CUDA(cudaMallocAsync(&part, sizeof(double) * pb, c.st));
   count_launch();
   k_plaquette<<<pb, 128, 0, c.st>>>(G, c.Ud, part);
   c.check_launch("gen_gauge_device");
   std::vector<double> h(pb);
   QWSG_CUDA(cudaMemcpyAsync(h.data(), part, sizeof(double) * pb, cudaMemcpyDeviceToHost, c.st));
-  QWSG_CUDA(cudaFreeAsync(part, c.st));
+  if (!fits) QWSG_CUDA(cudaFreeAsync(part, c.st));
   QWSG_CUDA(cudaStreamSynchronize(c.st));
   c.fields_h_valid = false;
   double tot = 0;
