@@ -277,7 +277,9 @@ int qwsg_gen_source(double* S, const int L[4], unsigned long long seed, int kind
  *   dag   1 = the adjoint hopping (deo_dag_*, deo_dag_in.cc:64);
  *   clov  1 = multiply by the parity's A^-1 (dee_*);
  *   mode  0 out = hops, 1 out += factor*hops, 2 out = in0 + factor*hops
- *         (one_minus_*). */
+ *         (one_minus_*).
+ * deo and clv take no device memory of their own (capturable from the first
+ * call on). */
 int qwsg_set_parities(qwsg_lattice* lat, int pce, int pco);
 int qwsg_deo_d(qwsg_lattice* lat, double* out, const double* in, int pe, int which, int dag,
                int clov, int mode, double factor, const double* in0);

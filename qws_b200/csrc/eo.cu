@@ -11,14 +11,15 @@
 //   MODE   0 out = acc (__store_sc), 1 out += coef acc (__store_add_sc),
 //          2 out = in0 + coef acc (one_minus_*).
 //
-// The operators work on vectors and fields of one parity each, stored
-// compactly in the order e = x/2 + Lx/2 (y + Ly (z + Lz t)).  On the full
-// lattice's planes the two parities alternate along a row, so one parity's
-// 16-byte entries use half of every 32-byte sector; compact, every byte
-// fetched is used (FP64 normal operator at 24^3x48: 2.6 ms on full planes
-// walked in x order, 0.70 ms compact).  Full-plane vectors of
-// the API are gathered and scattered by eo_gather / eo_scatter, the fields
-// once per load.
+// Two forms.  The Schur operators and solvers work on
+// vectors and fields of one parity each, stored compactly in the order
+// e = x/2 + Lx/2 (y + Ly (z + Lz t)).  On the full lattice's planes the two
+// parities alternate along a row, so one parity's 16-byte entries use half of
+// every 32-byte sector; compact, every byte fetched is used (FP64 normal
+// operator at 24^3x48: 2.6 ms on full planes walked in x order, 0.67 ms
+// compact).  Full-plane vectors of the API are gathered and scattered by
+// eo_gather / eo_scatter, the fields once per load.  A single hop operator of
+// the API reads and writes the full planes as they are (k_eo_planes).
 //
 // A y/z/t hop reads the other parity's site at the same compressed index x/2
 // of the neighbouring row, also across a boundary, as the reference's face
@@ -63,15 +64,30 @@ __device__ __forceinline__ EoSite eo_site(const EoArgs<T>& a, int e) {
   return s;
 }
 
-template <typename T, int WHICH, int DAG, int MU, int DIR, typename R = typename Arith<T>::R>
+// v: the neighbour's spinor (directions x, y, z) or its two spins (t); u: the
+// link.  acc += the hop's contribution
+template <typename T, int DAG, int MU, int DIR, typename R = typename Arith<T>::R>
+__device__ __forceinline__ void eo_hop_with(const R u[18], const R v[24], bool t_edge, int tbc,
+                                            R acc[24]) {
+  constexpr int PD = DAG ? -DIR : DIR;  // projector / reconstruction of this hop
+  R h[12], r[12];
+  project<R, MU, PD>(v, h);
+  if (DIR > 0)
+    link_mul<R, false>(u, h, r);
+  else
+    link_mul<R, true>(u, h, r);
+  R f = 1;
+  if (MU == 3) {
+    f = 2;
+    if (t_edge) f = (R)(2 * tbc);
+  }
+  reconstruct<R, MU, PD>(r, acc, f);
+}
+
+template <typename T, int DAG, int MU, int DIR, typename R = typename Arith<T>::R>
 __device__ __forceinline__ void eo_hop(const EoArgs<T>& a, const EoSite& s, int e, R acc[24]) {
   const int nxh = a.G.L[0] >> 1;
   const int c = MU == 0 ? 2 * s.xh + s.odd : MU == 1 ? s.y : MU == 2 ? s.z : s.t;
-  if (WHICH != 3) {
-    const int box = a.box[MU], in_box = c % box;
-    const bool inner = DIR > 0 ? in_box != box - 1 : in_box != 0;
-    if (inner ? !(WHICH & 1) : !(WHICH & 2)) return;
-  }
   int en = e;
   if (MU == 0) {
     // x+1 of an even x and x-1 of an odd x have the same compressed index
@@ -83,33 +99,22 @@ __device__ __forceinline__ void eo_hop(const EoArgs<T>& a, const EoSite& s, int 
     en = DIR > 0 ? (c + 1 == L ? e - (L - 1) * str : e + str)
                  : (c == 0 ? e + (L - 1) * str : e - str);
   }
-  constexpr int PD = DAG ? -DIR : DIR;  // projector / reconstruction of this hop
-  R v[24];
+  R v[24], u[18];
   if (MU == 3)
-    IO<T>::load_half(a.src, a.pad, en, PD > 0, v);
+    IO<T>::load_half(a.src, a.pad, en, (DAG ? -DIR : DIR) > 0, v);
   else
     IO<T>::load_spinor(a.src, a.pad, en, v);
-  R h[12], r[12], u[18];
-  project<R, MU, PD>(v, h);
   // forward: this parity's own link, backward: the other parity's
   IO<T>::load_link(DIR > 0 ? a.U[0] : a.U[1], a.pad, MU, DIR > 0 ? e : en, u);
-  if (DIR > 0)
-    link_mul<R, false>(u, h, r);
-  else
-    link_mul<R, true>(u, h, r);
-  R f = 1;
-  if (MU == 3) {
-    f = 2;
-    if (DIR > 0 ? s.t == a.G.L[3] - 1 : s.t == 0) f = (R)(2 * a.G.tbc);
-  }
-  reconstruct<R, MU, PD>(r, acc, f);
+  eo_hop_with<T, DAG, MU, DIR>(u, v, DIR > 0 ? s.t == a.G.L[3] - 1 : s.t == 0, a.G.tbc, acc);
 }
 
 // Memory bound: per output site 8 links (1152 bytes in FP64, each link of the
 // lattice once per launch), A^-1, the source once and the result: 2112 bytes
 // in FP64, 118 us at 24^3x48, 0.91 of the measured copy rate.
-template <typename T, int WHICH, int DAG, int CLOV, int MODE>
-__device__ __forceinline__ void eo_body(const EoArgs<T>& a) {
+// FP64 at 128 registers (4 CTAs of 128 threads an SM), FP32 at 80 (6)
+template <typename T, int DAG, int CLOV, int MODE>
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) k_eo(const EoArgs<T> a) {
   using R = typename Arith<T>::R;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= a.G.Vh) return;
@@ -117,14 +122,14 @@ __device__ __forceinline__ void eo_body(const EoArgs<T>& a) {
   R acc[24];
 #pragma unroll
   for (int j = 0; j < 24; j++) acc[j] = 0;
-  eo_hop<T, WHICH, DAG, 0, +1>(a, s, e, acc);
-  eo_hop<T, WHICH, DAG, 0, -1>(a, s, e, acc);
-  eo_hop<T, WHICH, DAG, 1, +1>(a, s, e, acc);
-  eo_hop<T, WHICH, DAG, 1, -1>(a, s, e, acc);
-  eo_hop<T, WHICH, DAG, 2, +1>(a, s, e, acc);
-  eo_hop<T, WHICH, DAG, 2, -1>(a, s, e, acc);
-  eo_hop<T, WHICH, DAG, 3, +1>(a, s, e, acc);
-  eo_hop<T, WHICH, DAG, 3, -1>(a, s, e, acc);
+  eo_hop<T, DAG, 0, +1>(a, s, e, acc);
+  eo_hop<T, DAG, 0, -1>(a, s, e, acc);
+  eo_hop<T, DAG, 1, +1>(a, s, e, acc);
+  eo_hop<T, DAG, 1, -1>(a, s, e, acc);
+  eo_hop<T, DAG, 2, +1>(a, s, e, acc);
+  eo_hop<T, DAG, 2, -1>(a, s, e, acc);
+  eo_hop<T, DAG, 3, +1>(a, s, e, acc);
+  eo_hop<T, DAG, 3, -1>(a, s, e, acc);
   if (CLOV) clover_apply<T>(a.C, a.pad, e, acc);
   if (MODE == 2) {
     R o[24];
@@ -134,10 +139,78 @@ __device__ __forceinline__ void eo_body(const EoArgs<T>& a) {
   }
   IO<T>::store_spinor(a.out, a.pad, e, acc);
 }
-// FP64 at 128 registers (4 CTAs of 128 threads an SM), FP32 at 80 (6)
+
+// The same on the full planes.  Thread i takes the sites of parity pe among 2i
+// and 2i + 1 of the planes' order: one, where the two are neighbours along an
+// even row, so that a warp reads runs of the planes.  Half of every sector is
+// still the other parity's, but the neighbouring warps' hops use it from L2.
+// Time of one operator at 24^3x48 (hops alone / with A^-1), against threads in
+// x order and against a gather, k_eo on copies that exist, and a scatter:
+// FP64 164 / 215 us (373 / 562; 203 / 227), FP32 75 / 105 (230 / 286; 98 / 109);
+// at 8^3x16 10 us (19 / 21; 17).
+template <typename T, int WHICH, int DAG, int MU, int DIR, typename R = typename Arith<T>::R>
+__device__ __forceinline__ void eo_hop_planes(const EoArgs<T>& a, const int x[4], int g, R acc[24]) {
+  const int L = a.G.L[MU];
+  if (WHICH != 3) {
+    const int box = a.box[MU], in_box = x[MU] % box;
+    const bool inner = DIR > 0 ? in_box != box - 1 : in_box != 0;
+    if (inner ? !(WHICH & 1) : !(WHICH & 2)) return;
+  }
+  int xn[4] = {x[0], x[1], x[2], x[3]};
+  xn[MU] = DIR > 0 ? (x[MU] + 1 == L ? 0 : x[MU] + 1) : (x[MU] == 0 ? L - 1 : x[MU] - 1);
+  if (MU > 0) xn[0] = 2 * (x[0] >> 1) + ((1 - a.pe + xn[1] + xn[2] + xn[3]) & 1);
+  const int gn = dd_index(a.G, xn);
+  R v[24], u[18];
+  if (MU == 3)
+    IO<T>::load_half(a.src, a.G.pad, gn, (DAG ? -DIR : DIR) > 0, v);
+  else
+    IO<T>::load_spinor(a.src, a.G.pad, gn, v);
+  IO<T>::load_link(a.U[0], a.G.pad, MU, DIR > 0 ? g : gn, u);
+  eo_hop_with<T, DAG, MU, DIR>(u, v, DIR > 0 ? x[3] == L - 1 : x[3] == 0, a.G.tbc, acc);
+}
 template <typename T, int WHICH, int DAG, int CLOV, int MODE>
-__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) k_eo(const EoArgs<T> a) {
-  eo_body<T, WHICH, DAG, CLOV, MODE>(a);
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) k_eo_planes(const EoArgs<T> a) {
+  using R = typename Arith<T>::R;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (2 * i >= a.G.V) return;
+  int x[4], x1[4];
+  site_coords(a.G, 2 * i, x);
+  site_coords(a.G, 2 * i + 1, x1);
+  const bool first = ((x[0] + x[1] + x[2] + x[3]) & 1) == a.pe;
+  bool second = ((x1[0] + x1[1] + x1[2] + x1[3]) & 1) == a.pe;
+  if (!first && !second) return;
+  int g = 2 * i;
+  if (!first) {
+    g++;
+#pragma unroll
+    for (int k = 0; k < 4; k++) x[k] = x1[k];
+    second = false;
+  }
+  for (;;) {
+    R acc[24];
+#pragma unroll
+    for (int j = 0; j < 24; j++) acc[j] = 0;
+    eo_hop_planes<T, WHICH, DAG, 0, +1>(a, x, g, acc);
+    eo_hop_planes<T, WHICH, DAG, 0, -1>(a, x, g, acc);
+    eo_hop_planes<T, WHICH, DAG, 1, +1>(a, x, g, acc);
+    eo_hop_planes<T, WHICH, DAG, 1, -1>(a, x, g, acc);
+    eo_hop_planes<T, WHICH, DAG, 2, +1>(a, x, g, acc);
+    eo_hop_planes<T, WHICH, DAG, 2, -1>(a, x, g, acc);
+    eo_hop_planes<T, WHICH, DAG, 3, +1>(a, x, g, acc);
+    eo_hop_planes<T, WHICH, DAG, 3, -1>(a, x, g, acc);
+    if (CLOV) clover_apply<T>(a.C, a.G.pad, g, acc);
+    if (MODE != 0) {
+      R o[24];
+      IO<T>::load_spinor(MODE == 1 ? a.out : a.in0, a.G.pad, g, o);
+#pragma unroll
+      for (int j = 0; j < 24; j++) acc[j] = o[j] + acc[j] * a.coef;
+    }
+    IO<T>::store_spinor(a.out, a.G.pad, g, acc);
+    if (!second) return;
+    second = false;  // (rows of odd length)
+    g++;
+    site_coords(a.G, g, x);
+  }
 }
 
 // out = A^-1 in on compact vectors (as an epilogue of the operator before it,
@@ -184,11 +257,11 @@ __global__ void __launch_bounds__(128) k_eo_gather(Geom G, T* __restrict__ dst, 
   IO<T>::load_spinor(src, G.pad, dd_index(G, x), v);
   IO<T>::store_spinor(dst, pad, e, v);
 }
-// compact vector -> parity pe of full planes: MODE 0 out = v, 1 out += coef v,
-// 2 out = in0 + coef v; ZERO: the other parity becomes zero (else untouched)
-template <typename T, int MODE, bool ZERO>
+// compact vector -> parity pe of full planes; ZERO: the other parity becomes
+// zero (else untouched)
+template <typename T, bool ZERO>
 __global__ void __launch_bounds__(128) k_eo_scatter(Geom G, T* out, const T* __restrict__ v, int pad,
-                                                    const T* in0, T coef, int pe) {
+                                                    int pe) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= G.V) return;
   int x[4];
@@ -199,16 +272,7 @@ __global__ void __launch_bounds__(128) k_eo_scatter(Geom G, T* out, const T* __r
 #pragma unroll
     for (int j = 0; j < 24; j++) o[j] = 0;
   } else {
-    T a[24];
-    IO<T>::load_spinor(v, pad, eo_index(G, x), a);
-    if (MODE == 0) {
-#pragma unroll
-      for (int j = 0; j < 24; j++) o[j] = a[j];
-    } else {
-      IO<T>::load_spinor(MODE == 1 ? out : in0, G.pad, g, o);
-#pragma unroll
-      for (int j = 0; j < 24; j++) o[j] = o[j] + a[j] * coef;
-    }
+    IO<T>::load_spinor(v, pad, eo_index(G, x), o);
   }
   IO<T>::store_spinor(out, G.pad, g, o);
 }
@@ -257,18 +321,14 @@ void eo_gather(const Geom& G, T* dst, int pad, const T* src, int pe, cudaStream_
   k_eo_gather<T><<<(G.Vh + 127) / 128, 128, 0, st>>>(G, dst, pad, src, pe);
 }
 template <typename T>
-void eo_scatter(const Geom& G, T* out, const T* v, int pad, int pe, int mode, T coef, const T* in0,
-                bool zero_other, cudaStream_t st) {
+void eo_scatter(const Geom& G, T* out, const T* v, int pad, int pe, bool zero_other,
+                cudaStream_t st) {
   const int nb = (G.V + 127) / 128;
   count_launch();
-  if (mode == 1)
-    k_eo_scatter<T, 1, false><<<nb, 128, 0, st>>>(G, out, v, pad, in0, coef, pe);
-  else if (mode == 2)
-    k_eo_scatter<T, 2, false><<<nb, 128, 0, st>>>(G, out, v, pad, in0, coef, pe);
-  else if (zero_other)
-    k_eo_scatter<T, 0, true><<<nb, 128, 0, st>>>(G, out, v, pad, in0, coef, pe);
+  if (zero_other)
+    k_eo_scatter<T, true><<<nb, 128, 0, st>>>(G, out, v, pad, pe);
   else
-    k_eo_scatter<T, 0, false><<<nb, 128, 0, st>>>(G, out, v, pad, in0, coef, pe);
+    k_eo_scatter<T, false><<<nb, 128, 0, st>>>(G, out, v, pad, pe);
 }
 template <typename T>
 void launch_clv(const Geom& G, T* out, const T* in, const T* C, int pe, cudaStream_t st) {
@@ -281,36 +341,46 @@ void launch_eo_clv(const EoArgs<T>& a, cudaStream_t st) {
   k_eo_clv<T><<<(a.G.Vh + 127) / 128, 128, 0, st>>>(a);
 }
 
-template <typename T, int WHICH, int DAG, int CLOV, int MODE>
-static void go(const EoArgs<T>& a, cudaStream_t st) {
-  count_launch();
-  k_eo<T, WHICH, DAG, CLOV, MODE><<<(a.G.Vh + 127) / 128, 128, 0, st>>>(a);
+template <typename T>
+void launch_eo(int dag, int clov, int mode, const EoArgs<T>& a, cudaStream_t st) {
+#define QWSG_EO(D, C, M)                                     \
+  if (dag == D && clov == C && mode == M) {                  \
+    count_launch();                                          \
+    k_eo<T, D, C, M><<<(a.G.Vh + 127) / 128, 128, 0, st>>>(a); \
+    return;                                                  \
+  }
+  QWSG_EO(0, 1, 0) QWSG_EO(1, 1, 0) QWSG_EO(0, 1, 2) QWSG_EO(1, 0, 2)
+#undef QWSG_EO
+  throw_unsupported_eo();
 }
 
-// compact vectors: mode 0, or 2 for the two forms of the Schur operators
 template <typename T>
-void launch_eo(int which, int dag, int clov, int mode, const EoArgs<T>& a, cudaStream_t st) {
-#define QWSG_EO(W, D, C, M)                                    \
-  if (which == W && dag == D && clov == C && mode == M) {      \
-    go<T, W, D, C, M>(a, st);                                  \
-    return;                                                    \
+void launch_eo_planes(int which, int dag, int clov, int mode, const EoArgs<T>& a, cudaStream_t st) {
+  // every combination the reference uses (12 FP64, 5 FP32 entry points); as
+  // many pairs of sites as sites of a parity
+#define QWSG_EO(W, D, C, M)                                               \
+  if (which == W && dag == D && clov == C && mode == M) {                 \
+    count_launch();                                                       \
+    k_eo_planes<T, W, D, C, M><<<(a.G.Vh + 127) / 128, 128, 0, st>>>(a);  \
+    return;                                                               \
   }
   QWSG_EO(1, 0, 0, 0) QWSG_EO(1, 0, 1, 0) QWSG_EO(1, 1, 0, 0) QWSG_EO(1, 1, 1, 0)
-  QWSG_EO(2, 0, 0, 0) QWSG_EO(2, 0, 1, 0) QWSG_EO(2, 1, 0, 0) QWSG_EO(2, 1, 1, 0)
+  QWSG_EO(1, 0, 1, 2) QWSG_EO(1, 1, 0, 2)
+  QWSG_EO(2, 0, 0, 1) QWSG_EO(2, 1, 0, 1) QWSG_EO(2, 0, 1, 1) QWSG_EO(2, 1, 1, 1)
   QWSG_EO(3, 0, 0, 0) QWSG_EO(3, 0, 1, 0) QWSG_EO(3, 1, 0, 0) QWSG_EO(3, 1, 1, 0)
-  QWSG_EO(3, 0, 1, 2) QWSG_EO(3, 1, 0, 2)
+  QWSG_EO(3, 0, 1, 2) QWSG_EO(3, 1, 0, 2) QWSG_EO(3, 0, 0, 1) QWSG_EO(3, 0, 1, 1)
 #undef QWSG_EO
   throw_unsupported_eo();
 }
 
 #define QWSG_INST(T)                                                                          \
-  template void launch_eo<T>(int, int, int, int, const EoArgs<T>&, cudaStream_t);             \
+  template void launch_eo<T>(int, int, int, const EoArgs<T>&, cudaStream_t);                  \
+  template void launch_eo_planes<T>(int, int, int, int, const EoArgs<T>&, cudaStream_t);      \
   template void launch_eo_clv<T>(const EoArgs<T>&, cudaStream_t);                             \
   template void launch_clv<T>(const Geom&, T*, const T*, const T*, int, cudaStream_t);        \
   template void eo_fields<T>(const Geom&, T*, T*, int, const T*, const T*, cudaStream_t);     \
   template void eo_gather<T>(const Geom&, T*, int, const T*, int, cudaStream_t);              \
-  template void eo_scatter<T>(const Geom&, T*, const T*, int, int, int, T, const T*, bool,    \
-                              cudaStream_t);
+  template void eo_scatter<T>(const Geom&, T*, const T*, int, int, bool, cudaStream_t);
 QWSG_INST(float)
 QWSG_INST(double)
 #undef QWSG_INST

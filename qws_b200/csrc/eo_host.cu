@@ -49,14 +49,6 @@ void Ctx::ensure_eo_s(int n) {
                    eoUs ? eoUs : Us, eoCs ? eoCs : Cs, eo_s, n);
 }
 
-template <typename R>
-static bool eo_loaded(const Ctx& c) {
-  if constexpr (std::is_same<R, double>::value)
-    return (c.eoUd || c.Ud) && (c.eoCd || c.Cd);
-  else
-    return (c.eoUs || c.Us) && (c.eoCs || c.Cs);
-}
-
 // the compact vectors as the BLAS kernels see them: one RHS of Vh sites
 static Geom eo_geom(const Ctx& c) {
   Geom G = c.G;
@@ -66,10 +58,23 @@ static Geom eo_geom(const Ctx& c) {
 }
 
 template <typename R>
-static EoArgs<R> eo_args(Ctx& c, int pe) {
+static EoArgs<R> eo_args(const Ctx& c, int pe) {
   EoArgs<R> a{};
   a.G = c.G;
   a.pad = c.eo_pad();
+  a.pe = pe;
+  // the reference's rank box: each rank holds two x-halves (NB = 2*npe0, ...)
+  a.box[0] = c.G.L[0] / (c.G.NB[0] / 2);
+  for (int mu = 1; mu < 4; mu++) a.box[mu] = c.G.L[mu] / c.G.NB[mu];
+  a.dxh = make_fastdiv(c.G.L[0] / 2);
+  a.dy = make_fastdiv(c.G.L[1]);
+  a.dz = make_fastdiv(c.G.L[2]);
+  return a;
+}
+// on the compact copies of the fields
+template <typename R>
+static EoArgs<R> eo_args_compact(const Ctx& c, int pe) {
+  EoArgs<R> a = eo_args<R>(c, pe);
   const R *U, *C;
   if constexpr (std::is_same<R, double>::value) {
     U = c.eoc_Ud;
@@ -82,27 +87,20 @@ static EoArgs<R> eo_args(Ctx& c, int pe) {
   a.U[0] = U + pe * par;
   a.U[1] = U + (1 - pe) * par;
   a.C = C + pe * par;
-  a.pe = pe;
-  // the reference's rank box: each rank holds two x-halves (NB = 2*npe0, ...)
-  a.box[0] = c.G.L[0] / (c.G.NB[0] / 2);
-  for (int mu = 1; mu < 4; mu++) a.box[mu] = c.G.L[mu] / c.G.NB[mu];
-  a.dxh = make_fastdiv(c.G.L[0] / 2);
-  a.dy = make_fastdiv(c.G.L[1]);
-  a.dz = make_fastdiv(c.G.L[2]);
   return a;
 }
 
-// one application on compact vectors (out: parity pe, in: the other; mode 0,
-// or 2: out = in0 + factor * hops)
+// one application of all hops on compact vectors (out: parity pe, in: the
+// other; mode 0, or 2: out = in0 + factor * hops)
 template <typename R>
-static void eo_apply(Ctx& c, R* out, const R* in, int pe, int which, int dag, int clov, int mode,
+static void eo_apply(Ctx& c, R* out, const R* in, int pe, int dag, int clov, int mode,
                      double factor, const R* in0) {
-  auto a = eo_args<R>(c, pe);
+  auto a = eo_args_compact<R>(c, pe);
   a.src = in;
   a.out = out;
   a.in0 = in0;
   a.coef = (R)factor;
-  launch_eo<R>(which, dag, clov, mode, a, c.st);
+  launch_eo<R>(dag, clov, mode, a, c.st);
 }
 
 template <typename R>
@@ -116,30 +114,28 @@ static R** eo_vecs(Ctx& c, int n) {
   }
 }
 
-// every combination the reference uses (12 FP64, 5 FP32 entry points)
-static bool eo_supported(int which, int dag, int clov, int mode) {
-  if (dag < 0 || dag > 1 || clov < 0 || clov > 1) return false;
-  switch (which) {
-    case 1: return mode == 0 || (mode == 2 && dag != clov);
-    case 2: return mode == 1;
-    case 3: return mode == 0 || (mode == 2 && dag != clov) || (mode == 1 && dag == 0);
-  }
-  return false;
-}
-
+// One operator of the API on the full planes as they are: no copy of the
+// fields and no work vector, so that a call on new fields, the first call on a
+// handle and one inside a stream capture cost what every call costs.
 template <typename R>
 void deo(Ctx& c, R* out, const R* in, int pe, int which, int dag, int clov, int mode,
          double factor, const R* in0) {
   if (pe != 0 && pe != 1) throw Error(1, "parity must be 0 or 1");
   if (mode == 2 && !in0) throw Error(1, "mode 2 needs in0");
-  if (!eo_supported(which, dag, clov, mode)) {
-    if (!eo_loaded<R>(c)) throw Error(4, "gauge/clover fields not loaded");
-    throw_unsupported_eo();
+  auto a = eo_args<R>(c, pe);
+  if constexpr (std::is_same<R, double>::value) {
+    a.U[0] = a.U[1] = c.eoUd ? c.eoUd : c.Ud;
+    a.C = c.eoCd ? c.eoCd : c.Cd;
+  } else {
+    a.U[0] = a.U[1] = c.eoUs ? c.eoUs : c.Us;
+    a.C = c.eoCs ? c.eoCs : c.Cs;
   }
-  R** v = eo_vecs<R>(c, 2);
-  eo_gather<R>(c.G, v[0], c.eo_pad(), in, 1 - pe, c.st);
-  eo_apply<R>(c, v[1], v[0], pe, which, dag, clov, 0, 0.0, nullptr);
-  eo_scatter<R>(c.G, out, v[1], c.eo_pad(), pe, mode, (R)factor, in0, false, c.st);
+  if (!a.U[0] || !a.C) throw Error(4, "gauge/clover fields not loaded");
+  a.src = in;
+  a.out = out;
+  a.in0 = in0;
+  a.coef = (R)factor;
+  launch_eo_planes<R>(which, dag, clov, mode, a, c.st);
   c.check_launch("deo");
 }
 template void deo<float>(Ctx&, float*, const float*, int, int, int, int, int, double, const float*);
@@ -164,17 +160,17 @@ template void clv<double>(Ctx&, double*, const double*, int);
 // (dee_deo_vm_(pco, pce) then one_minus_dee_deo_vm_(pce, pco)); compact, tmp
 // of the other parity
 static void mtilde_c(Ctx& c, double* out, const double* in, double* tmp) {
-  eo_apply<double>(c, tmp, in, c.pco, 3, 0, 1, 0, 0.0, nullptr);
-  eo_apply<double>(c, out, tmp, c.pce, 3, 0, 1, 2, -c.kappa * c.kappa, in);
+  eo_apply<double>(c, tmp, in, c.pco, 0, 1, 0, 0.0, nullptr);
+  eo_apply<double>(c, out, tmp, c.pce, 0, 1, 2, -c.kappa * c.kappa, in);
 }
 // mtilde_dag_vm_: clvd_vm2_(pce), dee_deo_dag_vm_(pco, pce), one_minus_deo_dag_vm_(pce, pco)
 static void mtilde_dag_c(Ctx& c, double* out, const double* in, double* t0, double* t1) {
-  auto a = eo_args<double>(c, c.pce);
+  auto a = eo_args_compact<double>(c, c.pce);
   a.src = in;
   a.out = t0;
   launch_eo_clv<double>(a, c.st);
-  eo_apply<double>(c, t1, t0, c.pco, 3, 1, 1, 0, 0.0, nullptr);
-  eo_apply<double>(c, out, t1, c.pce, 3, 1, 0, 2, -c.kappa * c.kappa, in);
+  eo_apply<double>(c, t1, t0, c.pco, 1, 1, 0, 0.0, nullptr);
+  eo_apply<double>(c, out, t1, c.pce, 1, 0, 2, -c.kappa * c.kappa, in);
 }
 // mtdagmt_vm_: mtilde_dag(mtilde(in)); work: eo_d[0 .. 2]
 static void mtdagmt_c(Ctx& c, double* out, const double* in) {
@@ -186,7 +182,7 @@ void mtilde_d(Ctx& c, double* out, const double* in) {
   double** v = eo_vecs<double>(c, 3);
   eo_gather<double>(c.G, v[1], c.eo_pad(), in, c.pce, c.st);
   mtilde_c(c, v[2], v[1], v[0]);
-  eo_scatter<double>(c.G, out, v[2], c.eo_pad(), c.pce, 0, 0.0, nullptr, false, c.st);
+  eo_scatter<double>(c.G, out, v[2], c.eo_pad(), c.pce, false, c.st);
   c.n_mtilde++;
   c.check_launch("mtilde_d");
 }
@@ -195,16 +191,16 @@ void mtilde_dag_d(Ctx& c, double* out, const double* in) {
   double** v = eo_vecs<double>(c, 4);
   eo_gather<double>(c.G, v[2], c.eo_pad(), in, c.pce, c.st);
   mtilde_dag_c(c, v[3], v[2], v[0], v[1]);
-  eo_scatter<double>(c.G, out, v[3], c.eo_pad(), c.pce, 0, 0.0, nullptr, false, c.st);
+  eo_scatter<double>(c.G, out, v[3], c.eo_pad(), c.pce, false, c.st);
   c.check_launch("mtilde_dag_d");
 }
 
 void mtilde_s(Ctx& c, float* out, const float* in) {
   float** v = eo_vecs<float>(c, 3);
   eo_gather<float>(c.G, v[1], c.eo_pad(), in, c.pce, c.st);
-  eo_apply<float>(c, v[0], v[1], c.pco, 3, 0, 1, 0, 0.0, nullptr);
-  eo_apply<float>(c, v[2], v[0], c.pce, 3, 0, 1, 2, -(double)(float)(c.kappa * c.kappa), v[1]);
-  eo_scatter<float>(c.G, out, v[2], c.eo_pad(), c.pce, 0, 0.0f, nullptr, false, c.st);
+  eo_apply<float>(c, v[0], v[1], c.pco, 0, 1, 0, 0.0, nullptr);
+  eo_apply<float>(c, v[2], v[0], c.pce, 0, 1, 2, -(double)(float)(c.kappa * c.kappa), v[1]);
+  eo_scatter<float>(c.G, out, v[2], c.eo_pad(), c.pce, false, c.st);
   c.check_launch("mtilde_s");
 }
 
@@ -245,7 +241,7 @@ int bicgstab_vm(Ctx& c, double* x, const double* b, int maxiter) {
     rho0 = rho;
     blas_bicg_p<double>(G, p, r, q, beta.real(), beta.imag(), omega.real(), omega.imag(), c.st);
   }
-  eo_scatter<double>(c.G, x, xx, G.pad, c.pce, 0, 0.0, nullptr, true, c.st);
+  eo_scatter<double>(c.G, x, xx, G.pad, c.pce, true, c.st);
   c.check_launch("bicgstab_vm");
   return iter;
 }
@@ -254,7 +250,7 @@ void mtdagmt_d(Ctx& c, double* out, const double* in) {
   double** v = eo_vecs<double>(c, 4);
   eo_gather<double>(c.G, v[3], c.eo_pad(), in, c.pce, c.st);
   mtdagmt_c(c, v[3], v[3]);  // (in is last read before out is written)
-  eo_scatter<double>(c.G, out, v[3], c.eo_pad(), c.pce, 0, 0.0, nullptr, false, c.st);
+  eo_scatter<double>(c.G, out, v[3], c.eo_pad(), c.pce, false, c.st);
   c.check_launch("mtdagmt_d");
 }
 
@@ -297,7 +293,7 @@ int cg_vm(Ctx& c, double* x, const double* b, int maxiter) {
     rho0 = rnorm;
     blas_bicg_p<double>(G, p, r, q, beta, 0.0, 0.0, 0.0, c.st);
   }
-  eo_scatter<double>(c.G, x, xx, G.pad, c.pce, 0, 0.0, nullptr, true, c.st);
+  eo_scatter<double>(c.G, x, xx, G.pad, c.pce, true, c.st);
   c.check_launch("cg_vm");
   return iter;
 }
@@ -377,8 +373,7 @@ int mcg_vm(Ctx& c, double* X, const double* b, int n, const double* sigma, int m
     alpha0 = alpha;
   }
   for (int k = 0; k < n; k++)
-    eo_scatter<double>(c.G, X + k * c.spinor_elems(), c.ms_x + k * ne, G.pad, c.pce, 0, 0.0, nullptr,
-                       true, c.st);
+    eo_scatter<double>(c.G, X + k * c.spinor_elems(), c.ms_x + k * ne, G.pad, c.pce, true, c.st);
   c.check_launch("mcg_vm");
   return iter;
 }

@@ -133,40 +133,42 @@ struct HopArgs {
 template <typename R>
 void launch_hop(int sel, int epi, const HopArgs<R>& a, cudaStream_t st);
 
-// even-odd (site parity) hopping on compact one-parity vectors, eo.cu.  T:
-// float or double; pad: the compact plane stride; parity p of a compact field
-// starts at p * 72 * pad reals.
+// even-odd (site parity) hopping, eo.cu.  T: float or double.  On compact
+// vectors parity p of a compact field starts at p * 72 * pad reals.
 template <typename T>
 struct EoArgs {
   Geom G;
-  const T* src;  // the other parity (launch_eo), or this one (launch_eo_clv)
+  const T* src;  // the other parity (launch_eo, launch_eo_planes), or this one (launch_eo_clv)
   const T* in0;
   T* out;
-  const T* U[2];  // links of parity pe and of the other
-  const T* C;     // A^-1 of parity pe
+  const T* U[2];  // links: compact those of parity pe and of the other, else the planes twice
+  const T* C;     // A^-1: compact that of parity pe
   T coef;
-  int pad;
+  int pad;     // plane stride of the compact vectors and fields
   int pe;      // parity of the output sites
   int box[4];  // the rank's local extents (inside / face classification)
   FastDiv dxh, dy, dz;
 };
-// (which, dag, clov) with mode 0, and the Schur operators' mode-2 forms
+// compact, all hops: the combinations of the Schur operators
 template <typename T>
-void launch_eo(int which, int dag, int clov, int mode, const EoArgs<T>& a, cudaStream_t st);
+void launch_eo(int dag, int clov, int mode, const EoArgs<T>& a, cudaStream_t st);
+// the full planes: every combination of the API
+template <typename T>
+void launch_eo_planes(int which, int dag, int clov, int mode, const EoArgs<T>& a, cudaStream_t st);
+// out = A^-1 in on compact vectors
 template <typename T>
 void launch_eo_clv(const EoArgs<T>& a, cudaStream_t st);
 // out = A^-1 in on the parity-pe sites of full planes
 template <typename T>
 void launch_clv(const Geom& G, T* out, const T* in, const T* C, int pe, cudaStream_t st);
-// full planes <-> compact; scatter modes 0 out = v, 1 out += coef v,
-// 2 out = in0 + coef v (mode 0 with zero_other: the other parity becomes 0)
+// full planes <-> compact; zero_other: the other parity becomes 0
 template <typename T>
 void eo_fields(const Geom& G, T* Ue, T* Ce, int pad, const T* U, const T* C, cudaStream_t st);
 template <typename T>
 void eo_gather(const Geom& G, T* dst, int pad, const T* src, int pe, cudaStream_t st);
 template <typename T>
-void eo_scatter(const Geom& G, T* out, const T* v, int pad, int pe, int mode, T coef, const T* in0,
-                bool zero_other, cudaStream_t st);
+void eo_scatter(const Geom& G, T* out, const T* v, int pad, int pe, bool zero_other,
+                cudaStream_t st);
 [[noreturn]] void throw_unsupported_eo();
 
 // ---------------------------------------------------------------------------

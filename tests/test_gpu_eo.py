@@ -184,3 +184,98 @@ def test_compact_fields_follow_changes():
         if child:
             child.close()
         lat.close()
+
+
+def fresh_lattice(L, NB, seed, csw=1.0, stream=None):
+    import qws_b200
+
+    lat = qws_b200.Lattice(L, NB, tbc=-1, kappa=0.12, stream=stream)
+    lat.gen_gauge_device(seed, 2, 0.36)
+    lat.build_clover(csw)
+    return lat
+
+
+def device_memory_of(f):
+    """bytes of device memory that f() took and kept (after a first run of
+    the same kernels elsewhere, which loads them)"""
+    import torch
+
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    f()
+    torch.cuda.synchronize()
+    return free - torch.cuda.mem_get_info()[0]
+
+
+def test_deo_takes_no_memory():
+    """One hop operator reads and writes the full planes: no copy of the
+    fields and no work vector, also on the handle's first call."""
+    import torch
+
+    L, NB = (16, 16, 16, 16), (2, 1, 1, 1)
+    taken = []
+    for _ in range(2):  # (the first handle loads the kernels)
+        lat = fresh_lattice(L, NB, 3)
+        x = {dt: lat.to_device(np.ones((lat.V, 24), dt)) for dt in (np.float64, np.float32)}
+        out = {dt: torch.zeros_like(v) for dt, v in x.items()}
+        taken.append(device_memory_of(lambda: [lat.deo(x[dt], 1, clov=1, out=out[dt]) for dt in x]))
+        lat.close()
+    assert taken[1] == 0
+
+
+def test_captured_deo_on_a_fresh_handle():
+    """The first call on a handle inside a stream capture; the replay reads the
+    fields as they are then."""
+    import qws_b200
+    import torch
+
+    L, NB = (8, 4, 4, 6), (2, 1, 1, 1)
+    st = torch.cuda.Stream()
+    lat = fresh_lattice(L, NB, 3, stream=st)
+    x = lat.to_device(qws_b200.gen_source(L, 4))
+    out = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        lat.deo(x, 1, clov=1, out=out)
+    for seed in (3, 5):
+        lat.gen_gauge_device(seed, 2, 0.36)
+        lat.build_clover(1.5)
+        g.replay()
+        torch.cuda.synchronize()
+        want = fresh_lattice(L, NB, seed, 1.5)
+        assert torch.equal(out, want.deo(x, 1, clov=1))
+        want.close()
+    lat.close()
+
+
+@pytest.mark.parametrize("L, NB", [((6, 5, 3, 2), (2, 1, 1, 1)), ((10, 6, 14, 4), (2, 2, 2, 2)),
+                                   ((10, 3, 3, 3), (2, 1, 1, 1)), ((4, 2, 2, 4), (2, 1, 1, 1))])
+@pytest.mark.parametrize("combo", [(0, 3, 0, 1, 0), (1, 1, 1, 0, 2), (0, 2, 0, 1, 1), (1, 3, 0, 0, 1)])
+def test_deo_at_edges(L, NB, combo):
+    """Rows of odd length (a pair of neighbouring sites of one parity, or none
+    of it), extents 2 and 3: FP64 1e-13 and FP32 1e-6 against the oracle, the
+    other parity of the output untouched."""
+    import qws_b200
+
+    U, _ = qws_b200.gen_gauge(L, 3, 2, 0.36)
+    C = qws_b200.gen_clover(U, L, 1.0, 0.12)
+    b, in0, acc0 = (qws_b200.gen_source(L, 4 + k) for k in range(3))
+    o = Oracle(L, NB, tbc=-1, kappa=0.12)
+    o.set_fields(U, C)
+    lat = qws_b200.Lattice(L, NB, tbc=-1, kappa=0.12)
+    lat.load_fields(U, C)
+    pe, which, dag, clov, mode = combo
+    m = parity_mask(L, pe)
+    try:
+        for dt, tol in ((np.float64, 1e-13), (np.float32, 1e-6)):
+            x, i0, a0 = b.astype(dt), in0.astype(dt), acc0.astype(dt)
+            ref = o.deo(x, pe, which, dag, clov, mode, dt(FAC), i0 if mode == 2 else None,
+                        out=a0.copy())
+            got = lat.to_host(lat.deo(lat.to_device(x), pe, which, dag, clov, mode, FAC,
+                                      in0=lat.to_device(i0) if mode == 2 else None,
+                                      out=lat.to_device(a0)))
+            assert rel(got, ref, m) < tol, (dt, combo)
+            assert np.array_equal(got[~m], a0[~m])
+    finally:
+        lat.close()
