@@ -191,8 +191,7 @@ struct Ctx {
   const float* eoCs = nullptr;
   int pce = 0, pco = 1;
   // compact one-parity copies of those fields (eo.cu), made on first use
-  // after every change of the fields they were made from, and work vectors
-  // of one parity each (24 * eo_pad() reals)
+  // after every change of the fields they were made from
   double* eoc_Ud = nullptr;
   double* eoc_Cd = nullptr;
   float* eoc_Us = nullptr;
@@ -204,17 +203,16 @@ struct Ctx {
   long eoc_gen_d = 0, eoc_gen_s = 0;
   static long next_fields_gen();
   int eo_pad() const { return (G.Vh + 127) / 128 * 128; }
-  static constexpr int kEoVecs = 9;
+  // work vectors of one parity each (24 * eo_pad() reals): the first
+  // kEoOpVecs and the FP32 ones the operators', the others the solvers'
+  static constexpr int kEoVecs = 9, kEoOpVecs = 4;
   double* eo_d[kEoVecs] = {};
-  float* eo_s[3] = {};
+  float* eo_s[2] = {};
   // multi-shift CG: the shifts' search vectors and solutions (ms_n compact
   // vectors each, back to back)
   double* ms_p = nullptr;
   double* ms_x = nullptr;
   int ms_n = 0;
-  // the compact fields and the first n work vectors
-  void ensure_eo_d(int n);
-  void ensure_eo_s(int n);
   long n_mtilde = 0;
 
   // CUDA graphs of the SAP preconditioner's launch sequences (about 40

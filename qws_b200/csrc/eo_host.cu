@@ -17,36 +17,76 @@ namespace qwsg {
   throw Error(2, "even-odd operator: unsupported combination of hop set / adjoint / clover / mode");
 }
 
-// each buffer on its own (a failed allocation is retried by the next call)
 template <typename R>
-static void eo_alloc(Ctx& c, R** p, size_t n) {
-  if (*p) return;
+static R* eo_alloc(Ctx& c, size_t n) {
   void* q = nullptr;
   QWSG_CUDA(cudaMalloc(&q, sizeof(R) * n));
   c.owned.push_back(q);
-  *p = static_cast<R*>(q);
   QWSG_CUDA(cudaMemsetAsync(q, 0, sizeof(R) * n, c.st));
+  return static_cast<R*>(q);
 }
+// The first n FP64 work vectors.  Those of the operators (four, and two in
+// FP32) come in one allocation on the first use of any of them: neighbouring
+// pairs also serve as one vector on the full planes (2 eo_pad() >= G.pad), and
+// a capture after that needs no more.
+static double** eo_work(Ctx& c, int n) {
+  const size_t ne = (size_t)24 * c.eo_pad();
+  if (!c.eo_d[0]) {
+    c.eo_d[0] = eo_alloc<double>(c, (Ctx::kEoOpVecs + 1) * ne);
+    for (int i = 1; i < Ctx::kEoOpVecs; i++) c.eo_d[i] = c.eo_d[0] + i * ne;
+    c.eo_s[0] = reinterpret_cast<float*>(c.eo_d[0] + Ctx::kEoOpVecs * ne);
+    c.eo_s[1] = c.eo_s[0] + ne;
+  }
+  if (n > Ctx::kEoOpVecs && !c.eo_d[Ctx::kEoOpVecs]) {  // the solvers'
+    c.eo_d[Ctx::kEoOpVecs] = eo_alloc<double>(c, (Ctx::kEoVecs - Ctx::kEoOpVecs) * ne);
+    for (int i = Ctx::kEoOpVecs + 1; i < Ctx::kEoVecs; i++)
+      c.eo_d[i] = c.eo_d[Ctx::kEoOpVecs] + (i - Ctx::kEoOpVecs) * ne;
+  }
+  return c.eo_d;
+}
+
+// Makes the compact copies of the fields follow the fields; false while the
+// handle's stream is being captured: a graph that held launches on the copies
+// would read them as they were at the capture, whatever the fields have become
+// by its replay, so captured operators read the fields on the full planes
+// (normal operator in FP64 at 24^3x48: 1.0 ms instead of 0.67).
 template <typename R>
-static void eo_ensure(Ctx& c, R** U, R** C, long& made, long gen, const R* srcU, const R* srcC,
-                      R** vecs, int n) {
+static bool eo_compact(Ctx& c) {
+  constexpr bool d = std::is_same<R, double>::value;
+  const R *srcU, *srcC;
+  R **U, **C;
+  long gen, *made;
+  const Ctx& owner = c.parent ? *c.parent : c;
+  if constexpr (d) {
+    srcU = c.eoUd ? c.eoUd : c.Ud;
+    srcC = c.eoCd ? c.eoCd : c.Cd;
+    U = &c.eoc_Ud;
+    C = &c.eoc_Cd;
+    gen = owner.fields_gen_d;
+    made = &c.eoc_gen_d;
+  } else {
+    srcU = c.eoUs ? c.eoUs : c.Us;
+    srcC = c.eoCs ? c.eoCs : c.Cs;
+    U = &c.eoc_Us;
+    C = &c.eoc_Cs;
+    gen = owner.fields_gen_s;
+    made = &c.eoc_gen_s;
+  }
   if (!srcU || !srcC) throw Error(4, "gauge/clover fields not loaded");
+  if (c.st != nullptr && c.st != cudaStreamLegacy) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    QWSG_CUDA(cudaStreamIsCapturing(c.st, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return false;
+  }
   const size_t pad = c.eo_pad();
-  eo_alloc(c, U, 144 * pad);
-  eo_alloc(c, C, 144 * pad);
-  for (int i = 0; i < n; i++) eo_alloc(c, vecs + i, 24 * pad);
-  if (made == gen) return;
-  eo_fields<R>(c.G, *U, *C, (int)pad, srcU, srcC, c.st);
-  c.check_launch("eo_fields");
-  made = gen;
-}
-void Ctx::ensure_eo_d(int n) {
-  eo_ensure<double>(*this, &eoc_Ud, &eoc_Cd, eoc_gen_d, (parent ? parent : this)->fields_gen_d,
-                    eoUd ? eoUd : Ud, eoCd ? eoCd : Cd, eo_d, n);
-}
-void Ctx::ensure_eo_s(int n) {
-  eo_ensure<float>(*this, &eoc_Us, &eoc_Cs, eoc_gen_s, (parent ? parent : this)->fields_gen_s,
-                   eoUs ? eoUs : Us, eoCs ? eoCs : Cs, eo_s, n);
+  if (!*U) *U = eo_alloc<R>(c, 144 * pad);
+  if (!*C) *C = eo_alloc<R>(c, 144 * pad);
+  if (*made != gen) {
+    eo_fields<R>(c.G, *U, *C, (int)pad, srcU, srcC, c.st);
+    c.check_launch("eo_fields");
+    *made = gen;
+  }
+  return true;
 }
 
 // the compact vectors as the BLAS kernels see them: one RHS of Vh sites
@@ -101,17 +141,6 @@ static void eo_apply(Ctx& c, R* out, const R* in, int pe, int dag, int clov, int
   a.in0 = in0;
   a.coef = (R)factor;
   launch_eo<R>(dag, clov, mode, a, c.st);
-}
-
-template <typename R>
-static R** eo_vecs(Ctx& c, int n) {
-  if constexpr (std::is_same<R, double>::value) {
-    c.ensure_eo_d(n);
-    return c.eo_d;
-  } else {
-    c.ensure_eo_s(n);
-    return c.eo_s;
-  }
 }
 
 // One operator of the API on the full planes as they are: no copy of the
@@ -178,29 +207,62 @@ static void mtdagmt_c(Ctx& c, double* out, const double* in) {
   mtilde_dag_c(c, out, c.eo_d[2], c.eo_d[0], c.eo_d[1]);
 }
 
+// the same on full planes; a work vector w holds both parities' intermediates
+template <typename R>
+static void mtilde_p(Ctx& c, R* out, const R* in, R* w, double coef) {
+  deo<R>(c, w, in, c.pco, 3, 0, 1, 0, 0.0, nullptr);
+  deo<R>(c, out, w, c.pce, 3, 0, 1, 2, coef, in);
+}
+static void mtilde_dag_p(Ctx& c, double* out, const double* in, double* w) {
+  clv<double>(c, w, in, c.pce);
+  deo<double>(c, w, w, c.pco, 3, 1, 1, 0, 0.0, nullptr);
+  deo<double>(c, out, w, c.pce, 3, 1, 0, 2, -c.kappa * c.kappa, in);
+}
+static void mtdagmt_p(Ctx& c, double* out, const double* in, double* w0, double* w1) {
+  mtilde_p<double>(c, w0, in, w0, -c.kappa * c.kappa);
+  mtilde_dag_p(c, out, w0, w1);
+}
+
 void mtilde_d(Ctx& c, double* out, const double* in) {
-  double** v = eo_vecs<double>(c, 3);
-  eo_gather<double>(c.G, v[1], c.eo_pad(), in, c.pce, c.st);
-  mtilde_c(c, v[2], v[1], v[0]);
-  eo_scatter<double>(c.G, out, v[2], c.eo_pad(), c.pce, false, c.st);
+  const bool compact = eo_compact<double>(c);
+  double** v = eo_work(c, 2);
+  if (compact) {
+    eo_gather<double>(c.G, v[1], c.eo_pad(), in, c.pce, c.st);
+    mtilde_c(c, v[1], v[1], v[0]);  // (in is last read where out is written)
+    eo_scatter<double>(c.G, out, v[1], c.eo_pad(), c.pce, false, c.st);
+  } else {
+    mtilde_p<double>(c, out, in, v[0], -c.kappa * c.kappa);
+  }
   c.n_mtilde++;
   c.check_launch("mtilde_d");
 }
 
 void mtilde_dag_d(Ctx& c, double* out, const double* in) {
-  double** v = eo_vecs<double>(c, 4);
-  eo_gather<double>(c.G, v[2], c.eo_pad(), in, c.pce, c.st);
-  mtilde_dag_c(c, v[3], v[2], v[0], v[1]);
-  eo_scatter<double>(c.G, out, v[3], c.eo_pad(), c.pce, false, c.st);
+  const bool compact = eo_compact<double>(c);
+  double** v = eo_work(c, 3);
+  if (compact) {
+    eo_gather<double>(c.G, v[2], c.eo_pad(), in, c.pce, c.st);
+    mtilde_dag_c(c, v[2], v[2], v[0], v[1]);
+    eo_scatter<double>(c.G, out, v[2], c.eo_pad(), c.pce, false, c.st);
+  } else {
+    mtilde_dag_p(c, out, in, v[0]);
+  }
   c.check_launch("mtilde_dag_d");
 }
 
 void mtilde_s(Ctx& c, float* out, const float* in) {
-  float** v = eo_vecs<float>(c, 3);
-  eo_gather<float>(c.G, v[1], c.eo_pad(), in, c.pce, c.st);
-  eo_apply<float>(c, v[0], v[1], c.pco, 0, 1, 0, 0.0, nullptr);
-  eo_apply<float>(c, v[2], v[0], c.pce, 0, 1, 2, -(double)(float)(c.kappa * c.kappa), v[1]);
-  eo_scatter<float>(c.G, out, v[2], c.eo_pad(), c.pce, false, c.st);
+  const bool compact = eo_compact<float>(c);
+  eo_work(c, 0);
+  float** v = c.eo_s;
+  const double coef = -(double)(float)(c.kappa * c.kappa);
+  if (compact) {
+    eo_gather<float>(c.G, v[1], c.eo_pad(), in, c.pce, c.st);
+    eo_apply<float>(c, v[0], v[1], c.pco, 0, 1, 0, 0.0, nullptr);
+    eo_apply<float>(c, v[1], v[0], c.pce, 0, 1, 2, coef, v[1]);
+    eo_scatter<float>(c.G, out, v[1], c.eo_pad(), c.pce, false, c.st);
+  } else {
+    mtilde_p<float>(c, out, in, v[0], coef);
+  }
   c.check_launch("mtilde_s");
 }
 
@@ -208,7 +270,8 @@ void mtilde_s(Ctx& c, float* out, const float* in) {
 // iter = 1..maxiter-1, converged when sqrt(|r|^2/|b|^2) < 1e-14 after the
 // omega step.  x: initial guess in, solution out.  Returns conviter.
 int bicgstab_vm(Ctx& c, double* x, const double* b, int maxiter) {
-  double** v = eo_vecs<double>(c, 8);
+  eo_compact<double>(c);
+  double** v = eo_work(c, 8);
   const Geom G = eo_geom(c);
   double *tmp = v[0], *bb = v[1], *q = v[2], *r = v[3], *p = v[4], *t = v[5], *r0 = v[6],
          *xx = v[7];
@@ -247,10 +310,15 @@ int bicgstab_vm(Ctx& c, double* x, const double* b, int maxiter) {
 }
 
 void mtdagmt_d(Ctx& c, double* out, const double* in) {
-  double** v = eo_vecs<double>(c, 4);
-  eo_gather<double>(c.G, v[3], c.eo_pad(), in, c.pce, c.st);
-  mtdagmt_c(c, v[3], v[3]);  // (in is last read before out is written)
-  eo_scatter<double>(c.G, out, v[3], c.eo_pad(), c.pce, false, c.st);
+  const bool compact = eo_compact<double>(c);
+  double** v = eo_work(c, 4);
+  if (compact) {
+    eo_gather<double>(c.G, v[3], c.eo_pad(), in, c.pce, c.st);
+    mtdagmt_c(c, v[3], v[3]);  // (in is last read before out is written)
+    eo_scatter<double>(c.G, out, v[3], c.eo_pad(), c.pce, false, c.st);
+  } else {
+    mtdagmt_p(c, out, in, v[0], v[2]);
+  }
   c.check_launch("mtdagmt_d");
 }
 
@@ -264,7 +332,8 @@ static void check_finite(double v, const char* what) {
 // (the reference does not report it).  A zero source returns x = 0 at
 // iteration 0 (the reference divides 0 by 0 there).
 int cg_vm(Ctx& c, double* x, const double* b, int maxiter) {
-  double** v = eo_vecs<double>(c, 9);
+  eo_compact<double>(c);
+  double** v = eo_work(c, 9);
   const Geom G = eo_geom(c);
   double *q = v[3], *r = v[4], *p = v[5], *r0 = v[6], *bb = v[7], *xx = v[8];
   eo_gather<double>(c.G, bb, G.pad, b, c.pce, c.st);
@@ -309,14 +378,15 @@ int cg_vm(Ctx& c, double* x, const double* b, int maxiter) {
 int mcg_vm(Ctx& c, double* X, const double* b, int n, const double* sigma, int maxiter) {
   if (n < 1 || n > Ctx::kMaxRhs) throw Error(1, "mcg_vm: number of shifts must be 1..32");
   if (c.G.nr != 1) throw Error(1, "mcg_vm: single right-hand side only");
-  double** v = eo_vecs<double>(c, 8);
+  eo_compact<double>(c);
+  double** v = eo_work(c, 8);
   const Geom G = eo_geom(c);
   const size_t ne = (size_t)24 * G.pad;
   if (c.ms_n < n) {
     c.ms_p = c.ms_x = nullptr;  // (the smaller ones stay with the handle)
     c.ms_n = 0;
-    eo_alloc(c, &c.ms_p, ne * n);
-    eo_alloc(c, &c.ms_x, ne * n);
+    c.ms_p = eo_alloc<double>(c, ne * n);
+    c.ms_x = eo_alloc<double>(c, ne * n);
     c.ms_n = n;
   }
   double *q = v[3], *r = v[4], *p = v[5], *r0 = v[6], *bb = v[7];

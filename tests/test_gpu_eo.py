@@ -279,3 +279,67 @@ def test_deo_at_edges(L, NB, combo):
             assert np.array_equal(got[~m], a0[~m])
     finally:
         lat.close()
+
+
+def schur_ops(lat, b):
+    """{name: (operator, input, output)} of the Schur operators"""
+    import torch
+
+    x = lat.to_device(b)
+    xs = lat.to_device(b.astype(np.float32))
+    ops = {"mtilde": lambda x, o: lat.mtilde(x, out=o),
+           "mtilde_dag": lambda x, o: lat.mtilde(x, dag=True, out=o),
+           "mtdagmt": lambda x, o: lat.mtdagmt(x, out=o)}
+    ops = {k: (f, x, torch.zeros_like(x)) for k, f in ops.items()}
+    ops["mtilde_s"] = (lambda x, o: lat.mtilde(x, out=o), xs, torch.zeros_like(xs))
+    return ops
+
+
+def close(a, b):
+    """two FP64 (FP32) results of the same sums, 8 hops and two 6x6 products
+    deep: 1e-14 (1e-6) relative"""
+    tol = 1e-14 if a.element_size() == 8 else 1e-6
+    return float((a - b).norm() / b.norm()) < tol
+
+
+@pytest.mark.parametrize("L, NB", [((8, 4, 4, 6), (2, 1, 1, 1)), ((10, 6, 14, 4), (2, 2, 2, 2))])
+def test_captured_schur_operators_follow_fields(L, NB):
+    """A graph captured after one call replays on the fields as they are then,
+    and a capture leaves nothing behind that the next plain call would take for
+    made."""
+    import qws_b200
+    import torch
+
+    st = torch.cuda.Stream()
+    b = qws_b200.gen_source(L, 4)
+    lat = fresh_lattice(L, NB, 3, stream=st)
+    ops = schur_ops(lat, b)
+    ops["mtilde"][0](*ops["mtilde"][1:])  # the first use makes the work vectors
+    torch.cuda.synchronize()
+    graphs = {}
+    for name, (f, x, out) in ops.items():
+        graphs[name] = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graphs[name], stream=st):
+            f(x, out)
+    for seed in (5, 7):
+        lat.gen_gauge_device(seed, 2, 0.36)
+        lat.build_clover(1.5)
+        want = fresh_lattice(L, NB, seed, 1.5)
+        for name, (f, x, out) in schur_ops(want, b).items():
+            f(x, out)
+            torch.cuda.synchronize()
+            graphs[name].replay()
+            torch.cuda.synchronize()
+            assert close(ops[name][2], out), (seed, name)
+        if seed == 5:  # captured after a change of the fields, before any plain call on them
+            g = torch.cuda.CUDAGraph()
+            f, x, out = ops["mtdagmt"]
+            with torch.cuda.graph(g, stream=st):
+                f(x, out)
+        for name, (f, x, out) in schur_ops(want, b).items():  # plain calls
+            f(x, out)
+            ops[name][0](*ops[name][1:])
+            torch.cuda.synchronize()
+            assert torch.equal(ops[name][2], out), (seed, name)
+        want.close()
+    lat.close()
