@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <complex>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -42,6 +43,18 @@ struct SolveStats {
   long inner_iters = 0;
   double rel_resid_recursive = 0;  // sqrt(|r|^2/|b|^2) at exit
   double rel_resid_true = -1;      // |b - D x| / |b| (when requested)
+};
+
+// compact copy of the gauge and clover fields (eo.cu): links of parity 0 and 1,
+// clover of parity 0 and 1, 72 * eo_pad() reals each
+template <typename R>
+struct EoCopy {
+  R* p;
+  long gen = 0;  // the state of the fields it was made from (0: not made yet)
+  explicit EoCopy(R* q) : p(q) {}
+  ~EoCopy() { cudaFree(p); }
+  EoCopy(const EoCopy&) = delete;
+  EoCopy& operator=(const EoCopy&) = delete;
 };
 
 struct Ctx {
@@ -190,22 +203,19 @@ struct Ctx {
   const float* eoUs = nullptr;
   const float* eoCs = nullptr;
   int pce = 0, pco = 1;
-  // compact one-parity copies of those fields (eo.cu), made on first use
-  // after every change of the fields they were made from
-  double* eoc_Ud = nullptr;
-  double* eoc_Cd = nullptr;
-  float* eoc_Us = nullptr;
-  float* eoc_Cs = nullptr;
-  // which state of the fields they were made from: every change of the
+  // compact copies of those fields, made on first use after every change of the
+  // fields, where memory holds them
+  std::shared_ptr<EoCopy<double>> eoc_d;
+  std::shared_ptr<EoCopy<float>> eoc_s;
+  // which state of the fields they follow (EoCopy::gen): every change of the
   // fields of a handle gives it a new number (unique in the process, so that
   // a borrowing handle sees its parent's changes and a change of parent)
   long fields_gen_d = next_fields_gen(), fields_gen_s = next_fields_gen();
-  long eoc_gen_d = 0, eoc_gen_s = 0;
   static long next_fields_gen();
   int eo_pad() const { return (G.Vh + 127) / 128 * 128; }
   // work vectors of one parity each (24 * eo_pad() reals): the first
   // kEoOpVecs and the FP32 ones the operators', the others the solvers'
-  static constexpr int kEoVecs = 9, kEoOpVecs = 4;
+  static constexpr int kEoVecs = 10, kEoOpVecs = 4;
   double* eo_d[kEoVecs] = {};
   float* eo_s[2] = {};
   // multi-shift CG: the shifts' search vectors and solutions (ms_n compact

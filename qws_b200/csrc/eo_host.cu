@@ -17,13 +17,27 @@ namespace qwsg {
   throw Error(2, "even-odd operator: unsupported combination of hop set / adjoint / clover / mode");
 }
 
-template <typename R>
-static R* eo_alloc(Ctx& c, size_t n) {
+static cudaError_t eo_try_alloc(void** p, size_t bytes) {
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();
+  return e;
+}
+// Work vectors come before copies of the fields: where memory holds only one
+// of the two, the copies go (the fields are then read on the full planes).
+static double* eo_alloc(Ctx& c, size_t n) {
   void* q = nullptr;
-  QWSG_CUDA(cudaMalloc(&q, sizeof(R) * n));
+  cudaError_t e = eo_try_alloc(&q, sizeof(double) * n);
+  if (e == cudaErrorMemoryAllocation && (c.eoc_d || c.eoc_s)) {
+    QWSG_CUDA(cudaDeviceSynchronize());
+    c.eoc_d.reset();
+    c.eoc_s.reset();
+    e = eo_try_alloc(&q, sizeof(double) * n);
+  }
+  if (e != cudaSuccess)
+    throw Error(3, std::string("even-odd work vectors: ") + cudaGetErrorString(e));
   c.owned.push_back(q);
-  QWSG_CUDA(cudaMemsetAsync(q, 0, sizeof(R) * n, c.st));
-  return static_cast<R*>(q);
+  QWSG_CUDA(cudaMemsetAsync(q, 0, sizeof(double) * n, c.st));
+  return static_cast<double*>(q);
 }
 // The first n FP64 work vectors.  Those of the operators (four, and two in
 // FP32) come in one allocation on the first use of any of them: neighbouring
@@ -32,61 +46,66 @@ static R* eo_alloc(Ctx& c, size_t n) {
 static double** eo_work(Ctx& c, int n) {
   const size_t ne = (size_t)24 * c.eo_pad();
   if (!c.eo_d[0]) {
-    c.eo_d[0] = eo_alloc<double>(c, (Ctx::kEoOpVecs + 1) * ne);
+    c.eo_d[0] = eo_alloc(c, (Ctx::kEoOpVecs + 1) * ne);
     for (int i = 1; i < Ctx::kEoOpVecs; i++) c.eo_d[i] = c.eo_d[0] + i * ne;
     c.eo_s[0] = reinterpret_cast<float*>(c.eo_d[0] + Ctx::kEoOpVecs * ne);
     c.eo_s[1] = c.eo_s[0] + ne;
   }
   if (n > Ctx::kEoOpVecs && !c.eo_d[Ctx::kEoOpVecs]) {  // the solvers'
-    c.eo_d[Ctx::kEoOpVecs] = eo_alloc<double>(c, (Ctx::kEoVecs - Ctx::kEoOpVecs) * ne);
+    c.eo_d[Ctx::kEoOpVecs] = eo_alloc(c, (Ctx::kEoVecs - Ctx::kEoOpVecs) * ne);
     for (int i = Ctx::kEoOpVecs + 1; i < Ctx::kEoVecs; i++)
       c.eo_d[i] = c.eo_d[Ctx::kEoOpVecs] + (i - Ctx::kEoOpVecs) * ne;
   }
   return c.eo_d;
 }
 
-// Makes the compact copies of the fields follow the fields; false while the
-// handle's stream is being captured: a graph that held launches on the copies
-// would read them as they were at the capture, whatever the fields have become
-// by its replay, so captured operators read the fields on the full planes
-// (normal operator in FP64 at 24^3x48: 1.0 ms instead of 0.67).
+// The compact copy of the fields, made to follow them.  Null, and the fields
+// are then read on the full planes (normal operator in FP64 at 24^3x48:
+// 0.95 ms instead of 0.67),
+//  - where device memory does not hold the copy (tried again by the next call);
+//  - while the handle's stream is being captured: a graph that held launches on
+//    the copy would read it as it was at the capture, whatever the fields have
+//    become by its replay.
 template <typename R>
-static bool eo_compact(Ctx& c) {
+static const R* eo_compact(Ctx& c) {
   constexpr bool d = std::is_same<R, double>::value;
-  const R *srcU, *srcC;
-  R **U, **C;
-  long gen, *made;
-  const Ctx& owner = c.parent ? *c.parent : c;
+  const R *U, *C;
   if constexpr (d) {
-    srcU = c.eoUd ? c.eoUd : c.Ud;
-    srcC = c.eoCd ? c.eoCd : c.Cd;
-    U = &c.eoc_Ud;
-    C = &c.eoc_Cd;
-    gen = owner.fields_gen_d;
-    made = &c.eoc_gen_d;
+    U = c.eoUd ? c.eoUd : c.Ud;
+    C = c.eoCd ? c.eoCd : c.Cd;
   } else {
-    srcU = c.eoUs ? c.eoUs : c.Us;
-    srcC = c.eoCs ? c.eoCs : c.Cs;
-    U = &c.eoc_Us;
-    C = &c.eoc_Cs;
-    gen = owner.fields_gen_s;
-    made = &c.eoc_gen_s;
+    U = c.eoUs ? c.eoUs : c.Us;
+    C = c.eoCs ? c.eoCs : c.Cs;
   }
-  if (!srcU || !srcC) throw Error(4, "gauge/clover fields not loaded");
+  if (!U || !C) throw Error(4, "gauge/clover fields not loaded");
   if (c.st != nullptr && c.st != cudaStreamLegacy) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     QWSG_CUDA(cudaStreamIsCapturing(c.st, &cs));
-    if (cs != cudaStreamCaptureStatusNone) return false;
+    if (cs != cudaStreamCaptureStatusNone) return nullptr;
   }
+  const Ctx& from = c.parent ? *c.parent : c;
+  const long gen = d ? from.fields_gen_d : from.fields_gen_s;
   const size_t pad = c.eo_pad();
-  if (!*U) *U = eo_alloc<R>(c, 144 * pad);
-  if (!*C) *C = eo_alloc<R>(c, 144 * pad);
-  if (*made != gen) {
-    eo_fields<R>(c.G, *U, *C, (int)pad, srcU, srcC, c.st);
-    c.check_launch("eo_fields");
-    *made = gen;
+  auto& copy = [&]() -> std::shared_ptr<EoCopy<R>>& {
+    if constexpr (d)
+      return c.eoc_d;
+    else
+      return c.eoc_s;
+  }();
+  if (!copy) {
+    void* q = nullptr;
+    const cudaError_t e = eo_try_alloc(&q, sizeof(R) * 288 * pad);
+    if (e == cudaErrorMemoryAllocation) return nullptr;
+    if (e != cudaSuccess)
+      throw Error(3, std::string("even-odd copy of the fields: ") + cudaGetErrorString(e));
+    copy = std::make_shared<EoCopy<R>>(static_cast<R*>(q));
   }
-  return true;
+  if (copy->gen != gen) {
+    eo_fields<R>(c.G, copy->p, copy->p + 144 * pad, (int)pad, U, C, c.st);
+    c.check_launch("eo_fields");
+    copy->gen = gen;
+  }
+  return copy->p;
 }
 
 // the compact vectors as the BLAS kernels see them: one RHS of Vh sites
@@ -111,31 +130,23 @@ static EoArgs<R> eo_args(const Ctx& c, int pe) {
   a.dz = make_fastdiv(c.G.L[2]);
   return a;
 }
-// on the compact copies of the fields
+// on a compact copy F of the fields
 template <typename R>
-static EoArgs<R> eo_args_compact(const Ctx& c, int pe) {
+static EoArgs<R> eo_args_compact(const Ctx& c, const R* F, int pe) {
   EoArgs<R> a = eo_args<R>(c, pe);
-  const R *U, *C;
-  if constexpr (std::is_same<R, double>::value) {
-    U = c.eoc_Ud;
-    C = c.eoc_Cd;
-  } else {
-    U = c.eoc_Us;
-    C = c.eoc_Cs;
-  }
   const size_t par = (size_t)72 * a.pad;
-  a.U[0] = U + pe * par;
-  a.U[1] = U + (1 - pe) * par;
-  a.C = C + pe * par;
+  a.U[0] = F + pe * par;
+  a.U[1] = F + (1 - pe) * par;
+  a.C = F + (2 + pe) * par;
   return a;
 }
 
 // one application of all hops on compact vectors (out: parity pe, in: the
 // other; mode 0, or 2: out = in0 + factor * hops)
 template <typename R>
-static void eo_apply(Ctx& c, R* out, const R* in, int pe, int dag, int clov, int mode,
+static void eo_apply(Ctx& c, const R* F, R* out, const R* in, int pe, int dag, int clov, int mode,
                      double factor, const R* in0) {
-  auto a = eo_args_compact<R>(c, pe);
+  auto a = eo_args_compact<R>(c, F, pe);
   a.src = in;
   a.out = out;
   a.in0 = in0;
@@ -186,28 +197,30 @@ template void clv<float>(Ctx&, float*, const float*, int);
 template void clv<double>(Ctx&, double*, const double*, int);
 
 // mtilde_vm_: out_e = in_e - kappa^2 A_ee^-1 H_eo A_oo^-1 H_oe in_e
-// (dee_deo_vm_(pco, pce) then one_minus_dee_deo_vm_(pce, pco)); compact, tmp
-// of the other parity
-static void mtilde_c(Ctx& c, double* out, const double* in, double* tmp) {
-  eo_apply<double>(c, tmp, in, c.pco, 0, 1, 0, 0.0, nullptr);
-  eo_apply<double>(c, out, tmp, c.pce, 0, 1, 2, -c.kappa * c.kappa, in);
+// (dee_deo_vm_(pco, pce) then one_minus_dee_deo_vm_(pce, pco)); compact, on the
+// copy F of the fields, tmp of the other parity; out may be in
+static void mtilde_c(Ctx& c, const double* F, double* out, const double* in, double* tmp) {
+  eo_apply<double>(c, F, tmp, in, c.pco, 0, 1, 0, 0.0, nullptr);
+  eo_apply<double>(c, F, out, tmp, c.pce, 0, 1, 2, -c.kappa * c.kappa, in);
 }
 // mtilde_dag_vm_: clvd_vm2_(pce), dee_deo_dag_vm_(pco, pce), one_minus_deo_dag_vm_(pce, pco)
-static void mtilde_dag_c(Ctx& c, double* out, const double* in, double* t0, double* t1) {
-  auto a = eo_args_compact<double>(c, c.pce);
+static void mtilde_dag_c(Ctx& c, const double* F, double* out, const double* in, double* t0,
+                         double* t1) {
+  auto a = eo_args_compact<double>(c, F, c.pce);
   a.src = in;
   a.out = t0;
   launch_eo_clv<double>(a, c.st);
-  eo_apply<double>(c, t1, t0, c.pco, 1, 1, 0, 0.0, nullptr);
-  eo_apply<double>(c, out, t1, c.pce, 1, 0, 2, -c.kappa * c.kappa, in);
+  eo_apply<double>(c, F, t1, t0, c.pco, 1, 1, 0, 0.0, nullptr);
+  eo_apply<double>(c, F, out, t1, c.pce, 1, 0, 2, -c.kappa * c.kappa, in);
 }
-// mtdagmt_vm_: mtilde_dag(mtilde(in)); work: eo_d[0 .. 2]
-static void mtdagmt_c(Ctx& c, double* out, const double* in) {
-  mtilde_c(c, c.eo_d[2], in, c.eo_d[0]);
-  mtilde_dag_c(c, out, c.eo_d[2], c.eo_d[0], c.eo_d[1]);
+// mtdagmt_vm_ (qws.cc:566-571): mtilde_dag(mtilde(in)); work: eo_d[0 .. 2]
+static void mtdagmt_c(Ctx& c, const double* F, double* out, const double* in) {
+  mtilde_c(c, F, c.eo_d[2], in, c.eo_d[0]);
+  mtilde_dag_c(c, F, out, c.eo_d[2], c.eo_d[0], c.eo_d[1]);
 }
 
-// the same on full planes; a work vector w holds both parities' intermediates
+// the same on full planes; a work vector holds both parities' intermediates
+// (mtilde_p: out may be in, or w; mtdagmt_p: in may be w0, out w1 or in)
 template <typename R>
 static void mtilde_p(Ctx& c, R* out, const R* in, R* w, double coef) {
   deo<R>(c, w, in, c.pco, 3, 0, 1, 0, 0.0, nullptr);
@@ -219,16 +232,33 @@ static void mtilde_dag_p(Ctx& c, double* out, const double* in, double* w) {
   deo<double>(c, out, w, c.pce, 3, 1, 0, 2, -c.kappa * c.kappa, in);
 }
 static void mtdagmt_p(Ctx& c, double* out, const double* in, double* w0, double* w1) {
-  mtilde_p<double>(c, w0, in, w0, -c.kappa * c.kappa);
-  mtilde_dag_p(c, out, w0, w1);
+  deo<double>(c, w0, in, c.pco, 3, 0, 1, 0, 0.0, nullptr);
+  deo<double>(c, w1, w0, c.pce, 3, 0, 1, 2, -c.kappa * c.kappa, in);
+  mtilde_dag_p(c, out, w1, w0);
+}
+
+// the solvers' operators: compact vectors in and out, on a compact copy F of
+// the fields or (null) on the full planes; work: eo_d[0, 1] and eo_d[0 .. 3]
+static void solve_mtilde(Ctx& c, const double* F, double* out, const double* in) {
+  double* w = c.eo_d[0];
+  if (F) return mtilde_c(c, F, out, in, w);
+  eo_scatter<double>(c.G, w, in, c.eo_pad(), c.pce, false, c.st);
+  mtilde_p<double>(c, w, w, w, -c.kappa * c.kappa);
+  eo_gather<double>(c.G, out, c.eo_pad(), w, c.pce, c.st);
+}
+static void solve_mtdagmt(Ctx& c, const double* F, double* out, const double* in) {
+  if (F) return mtdagmt_c(c, F, out, in);
+  double *w0 = c.eo_d[0], *w1 = c.eo_d[2];
+  eo_scatter<double>(c.G, w0, in, c.eo_pad(), c.pce, false, c.st);
+  mtdagmt_p(c, w1, w0, w0, w1);
+  eo_gather<double>(c.G, out, c.eo_pad(), w1, c.pce, c.st);
 }
 
 void mtilde_d(Ctx& c, double* out, const double* in) {
-  const bool compact = eo_compact<double>(c);
   double** v = eo_work(c, 2);
-  if (compact) {
+  if (const double* F = eo_compact<double>(c)) {
     eo_gather<double>(c.G, v[1], c.eo_pad(), in, c.pce, c.st);
-    mtilde_c(c, v[1], v[1], v[0]);  // (in is last read where out is written)
+    mtilde_c(c, F, v[1], v[1], v[0]);
     eo_scatter<double>(c.G, out, v[1], c.eo_pad(), c.pce, false, c.st);
   } else {
     mtilde_p<double>(c, out, in, v[0], -c.kappa * c.kappa);
@@ -238,11 +268,10 @@ void mtilde_d(Ctx& c, double* out, const double* in) {
 }
 
 void mtilde_dag_d(Ctx& c, double* out, const double* in) {
-  const bool compact = eo_compact<double>(c);
   double** v = eo_work(c, 3);
-  if (compact) {
+  if (const double* F = eo_compact<double>(c)) {
     eo_gather<double>(c.G, v[2], c.eo_pad(), in, c.pce, c.st);
-    mtilde_dag_c(c, v[2], v[2], v[0], v[1]);
+    mtilde_dag_c(c, F, v[2], v[2], v[0], v[1]);
     eo_scatter<double>(c.G, out, v[2], c.eo_pad(), c.pce, false, c.st);
   } else {
     mtilde_dag_p(c, out, in, v[0]);
@@ -251,14 +280,13 @@ void mtilde_dag_d(Ctx& c, double* out, const double* in) {
 }
 
 void mtilde_s(Ctx& c, float* out, const float* in) {
-  const bool compact = eo_compact<float>(c);
   eo_work(c, 0);
   float** v = c.eo_s;
   const double coef = -(double)(float)(c.kappa * c.kappa);
-  if (compact) {
+  if (const float* F = eo_compact<float>(c)) {
     eo_gather<float>(c.G, v[1], c.eo_pad(), in, c.pce, c.st);
-    eo_apply<float>(c, v[0], v[1], c.pco, 0, 1, 0, 0.0, nullptr);
-    eo_apply<float>(c, v[1], v[0], c.pce, 0, 1, 2, coef, v[1]);
+    eo_apply<float>(c, F, v[0], v[1], c.pco, 0, 1, 0, 0.0, nullptr);
+    eo_apply<float>(c, F, v[1], v[0], c.pce, 0, 1, 2, coef, v[1]);
     eo_scatter<float>(c.G, out, v[1], c.eo_pad(), c.pce, false, c.st);
   } else {
     mtilde_p<float>(c, out, in, v[0], coef);
@@ -266,32 +294,43 @@ void mtilde_s(Ctx& c, float* out, const float* in) {
   c.check_launch("mtilde_s");
 }
 
+void mtdagmt_d(Ctx& c, double* out, const double* in) {
+  double** v = eo_work(c, 4);
+  if (const double* F = eo_compact<double>(c)) {
+    eo_gather<double>(c.G, v[3], c.eo_pad(), in, c.pce, c.st);
+    mtdagmt_c(c, F, v[3], v[3]);
+    eo_scatter<double>(c.G, out, v[3], c.eo_pad(), c.pce, false, c.st);
+  } else {
+    mtdagmt_p(c, out, in, v[0], v[2]);
+  }
+  c.check_launch("mtdagmt_d");
+}
+
 // bicgstab_vm_ (bicgstab.cc:68-333): BiCGStab on mtilde for the pce parity,
 // iter = 1..maxiter-1, converged when sqrt(|r|^2/|b|^2) < 1e-14 after the
 // omega step.  x: initial guess in, solution out.  Returns conviter.
 int bicgstab_vm(Ctx& c, double* x, const double* b, int maxiter) {
-  eo_compact<double>(c);
-  double** v = eo_work(c, 8);
+  double** v = eo_work(c, 9);
+  const double* F = eo_compact<double>(c);
   const Geom G = eo_geom(c);
-  double *tmp = v[0], *bb = v[1], *q = v[2], *r = v[3], *p = v[4], *t = v[5], *r0 = v[6],
-         *xx = v[7];
+  double *bb = v[2], *q = v[3], *r = v[4], *p = v[5], *t = v[6], *r0 = v[7], *xx = v[8];
   eo_gather<double>(c.G, bb, G.pad, b, c.pce, c.st);
   eo_gather<double>(c.G, xx, G.pad, x, c.pce, c.st);
-  mtilde_c(c, q, xx, tmp);
+  solve_mtilde(c, F, q, xx);
   blas_bicg_init<double>(G, bb, q, r, p, r0, c.d_res, c.rb, c.st);
   const double* h = c.fetch(2);
   const double bnorm = h[0];
   std::complex<double> rho0(h[1], 0), rho, beta, omega, alpha, ctmp;
   int iter;
   for (iter = 1; iter < maxiter; iter++) {
-    mtilde_c(c, q, p, tmp);
+    solve_mtilde(c, F, q, p);
     blas_cdot<double>(G, r0, q, c.d_res, c.rb, c.st);
     h = c.fetch(2);
     ctmp = std::complex<double>(h[0], h[1]);
     alpha = rho0 / ctmp;
     blas_bicg_update<double>(G, xx, r, p, q, alpha.real(), alpha.imag(), nullptr, c.d_res, c.rb,
                              c.st);
-    mtilde_c(c, t, r, tmp);
+    solve_mtilde(c, F, t, r);
     blas_norm_cdot<double>(G, t, r, c.d_res, c.rb, c.st);
     h = c.fetch(3);
     omega = std::complex<double>(h[1] / h[0], h[2] / h[0]);
@@ -309,19 +348,6 @@ int bicgstab_vm(Ctx& c, double* x, const double* b, int maxiter) {
   return iter;
 }
 
-void mtdagmt_d(Ctx& c, double* out, const double* in) {
-  const bool compact = eo_compact<double>(c);
-  double** v = eo_work(c, 4);
-  if (compact) {
-    eo_gather<double>(c.G, v[3], c.eo_pad(), in, c.pce, c.st);
-    mtdagmt_c(c, v[3], v[3]);  // (in is last read before out is written)
-    eo_scatter<double>(c.G, out, v[3], c.eo_pad(), c.pce, false, c.st);
-  } else {
-    mtdagmt_p(c, out, in, v[0], v[2]);
-  }
-  c.check_launch("mtdagmt_d");
-}
-
 static void check_finite(double v, const char* what) {
   if (!std::isfinite(v)) throw Error(3, std::string(what) + ": non-finite residual norm");
 }
@@ -332,13 +358,13 @@ static void check_finite(double v, const char* what) {
 // (the reference does not report it).  A zero source returns x = 0 at
 // iteration 0 (the reference divides 0 by 0 there).
 int cg_vm(Ctx& c, double* x, const double* b, int maxiter) {
-  eo_compact<double>(c);
-  double** v = eo_work(c, 9);
+  double** v = eo_work(c, 10);
+  const double* F = eo_compact<double>(c);
   const Geom G = eo_geom(c);
-  double *q = v[3], *r = v[4], *p = v[5], *r0 = v[6], *bb = v[7], *xx = v[8];
+  double *q = v[4], *r = v[5], *p = v[6], *r0 = v[7], *bb = v[8], *xx = v[9];
   eo_gather<double>(c.G, bb, G.pad, b, c.pce, c.st);
   eo_gather<double>(c.G, xx, G.pad, x, c.pce, c.st);
-  mtdagmt_c(c, q, xx);
+  solve_mtdagmt(c, F, q, xx);
   blas_bicg_init<double>(G, bb, q, r, p, r0, c.d_res, c.rb, c.st);
   const double* h = c.fetch(2);
   const double bnorm = h[0];
@@ -349,7 +375,7 @@ int cg_vm(Ctx& c, double* x, const double* b, int maxiter) {
   }
   int iter;
   for (iter = 1; iter < maxiter; iter++) {
-    mtdagmt_c(c, q, p);
+    solve_mtdagmt(c, F, q, p);
     blas_cdot<double>(G, p, q, c.d_res, c.rb, c.st);
     h = c.fetch(1);
     const double alpha = rho0 / h[0];
@@ -378,18 +404,18 @@ int cg_vm(Ctx& c, double* x, const double* b, int maxiter) {
 int mcg_vm(Ctx& c, double* X, const double* b, int n, const double* sigma, int maxiter) {
   if (n < 1 || n > Ctx::kMaxRhs) throw Error(1, "mcg_vm: number of shifts must be 1..32");
   if (c.G.nr != 1) throw Error(1, "mcg_vm: single right-hand side only");
-  eo_compact<double>(c);
-  double** v = eo_work(c, 8);
+  double** v = eo_work(c, 9);
   const Geom G = eo_geom(c);
   const size_t ne = (size_t)24 * G.pad;
   if (c.ms_n < n) {
     c.ms_p = c.ms_x = nullptr;  // (the smaller ones stay with the handle)
     c.ms_n = 0;
-    c.ms_p = eo_alloc<double>(c, ne * n);
-    c.ms_x = eo_alloc<double>(c, ne * n);
+    c.ms_p = eo_alloc(c, ne * n);
+    c.ms_x = eo_alloc(c, ne * n);
     c.ms_n = n;
   }
-  double *q = v[3], *r = v[4], *p = v[5], *r0 = v[6], *bb = v[7];
+  const double* F = eo_compact<double>(c);
+  double *q = v[4], *r = v[5], *p = v[6], *r0 = v[7], *bb = v[8];
   eo_gather<double>(c.G, bb, G.pad, b, c.pce, c.st);
   blas_bicg_init<double>(G, bb, nullptr, r, p, r0, c.d_res, c.rb, c.st);
   const double* h = c.fetch(1);
@@ -409,7 +435,7 @@ int mcg_vm(Ctx& c, double* X, const double* b, int n, const double* sigma, int m
   double alpha0 = 1.0, beta = 0.0;
   int iter;
   for (iter = 1; iter < maxiter; iter++) {
-    mtdagmt_c(c, q, p);
+    solve_mtdagmt(c, F, q, p);
     blas_cdot<double>(G, p, q, c.d_res, c.rb, c.st);
     h = c.fetch(1);
     const double alpha = -rho0 / h[0];

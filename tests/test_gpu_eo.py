@@ -343,3 +343,56 @@ def test_captured_schur_operators_follow_fields(L, NB):
             assert torch.equal(ops[name][2], out), (seed, name)
         want.close()
     lat.close()
+
+
+@pytest.mark.parametrize("bytes_a_site", [1450, 2000])
+def test_without_room_for_a_copy_of_the_fields(bytes_a_site):
+    """With that many bytes of device memory a site left, all operators and solvers
+    run, to the same results: 1,450 hold the work vectors (480 bytes a site of
+    the operators', 576 more of the solvers') but no copy of the fields (1,152
+    in FP64) beside them; 2,000 hold a copy until the solvers need their
+    vectors.  Once there is room again they use a copy."""
+    import qws_b200
+    import torch
+
+    L, NB = (16, 16, 16, 32), (2, 1, 1, 1)
+    b = qws_b200.gen_source(L, 4)
+    solvers = {"bicgstab": lambda l, x, d: l.bicgstab_vm(x, d, 200),
+               "cg": lambda l, x, d: l.cg_vm(x, d, 1000)}
+    runs = []
+    for scarce in (False, True):  # (the first handle loads the kernels)
+        lat = fresh_lattice(L, NB, 3)
+        ops, bd = schur_ops(lat, b), lat.to_device(b)
+        xs = {name: torch.zeros_like(bd) for name in solvers}
+        runs.append((ops, xs))
+        if not scarce:  # the kernels on full planes
+            lat.deo(bd, 0, clov=1)
+            for dag in (0, 1):
+                for mode, clov in ((0, 1), (2, 1 - dag)):
+                    lat.deo(bd, 0, dag=dag, clov=clov, mode=mode, in0=bd)
+                    lat.deo(bd.float(), 0, dag=dag, clov=clov, mode=mode, in0=bd.float())
+            lat.clv(bd, 0)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        fill, chunk, keep = [], 2 << 20, bytes_a_site * lat.V
+        while scarce and (free := torch.cuda.mem_get_info()[0]) > keep + chunk:
+            fill.append(torch.empty((free - keep) // chunk * chunk, dtype=torch.uint8, device="cuda"))
+        try:
+            for f, x, out in ops.values():
+                f(x, out)
+            for name, f in solvers.items():
+                f(lat, xs[name], bd)
+            torch.cuda.synchronize()
+        finally:
+            fill.clear()
+            torch.cuda.empty_cache()
+        if scarce:
+            for name in solvers:
+                assert float((xs[name] - runs[0][1][name]).norm() / xs[name].norm()) < 1e-11, name
+            for again in (False, True):
+                for name, (f, x, out) in ops.items():
+                    want = runs[0][0][name][2]
+                    assert torch.equal(out, want) if again else close(out, want), (name, again)
+                    f(x, out)
+                torch.cuda.synchronize()
+        lat.close()
