@@ -4,6 +4,7 @@
 
 #include <complex>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -52,7 +53,10 @@ struct EoCopy {
   R* p;
   long gen = 0;  // the state of the fields it was made from (0: not made yet)
   explicit EoCopy(R* q) : p(q) {}
-  ~EoCopy() { cudaFree(p); }
+  ~EoCopy() {
+    cudaDeviceSynchronize();  // (whichever streams still read it)
+    cudaFree(p);
+  }
   EoCopy(const EoCopy&) = delete;
   EoCopy& operator=(const EoCopy&) = delete;
 };
@@ -204,7 +208,9 @@ struct Ctx {
   const float* eoCs = nullptr;
   int pce = 0, pco = 1;
   // compact copies of those fields, made on first use after every change of the
-  // fields, where memory holds them
+  // fields, where memory holds them; a borrowing handle uses its parent's
+  std::mutex eo_mu;
+  bool release_copies();  // gives their memory back; false if there were none
   std::shared_ptr<EoCopy<double>> eoc_d;
   std::shared_ptr<EoCopy<float>> eoc_s;
   // which state of the fields they follow (EoCopy::gen): every change of the

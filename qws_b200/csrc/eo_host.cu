@@ -17,6 +17,17 @@ namespace qwsg {
   throw Error(2, "even-odd operator: unsupported combination of hop set / adjoint / clover / mode");
 }
 
+// whose copy of the fields a handle reads: that of the lattice they live on
+static Ctx& eo_owner(Ctx& c) { return c.parent ? *c.parent : c; }
+
+bool Ctx::release_copies() {
+  std::lock_guard<std::mutex> lk(eo_mu);
+  if (!eoc_d && !eoc_s) return false;
+  eoc_d.reset();
+  eoc_s.reset();
+  return true;
+}
+
 static cudaError_t eo_try_alloc(void** p, size_t bytes) {
   const cudaError_t e = cudaMalloc(p, bytes);
   if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();
@@ -27,12 +38,8 @@ static cudaError_t eo_try_alloc(void** p, size_t bytes) {
 static double* eo_alloc(Ctx& c, size_t n) {
   void* q = nullptr;
   cudaError_t e = eo_try_alloc(&q, sizeof(double) * n);
-  if (e == cudaErrorMemoryAllocation && (c.eoc_d || c.eoc_s)) {
-    QWSG_CUDA(cudaDeviceSynchronize());
-    c.eoc_d.reset();
-    c.eoc_s.reset();
+  if (e == cudaErrorMemoryAllocation && eo_owner(c).release_copies())
     e = eo_try_alloc(&q, sizeof(double) * n);
-  }
   if (e != cudaSuccess)
     throw Error(3, std::string("even-odd work vectors: ") + cudaGetErrorString(e));
   c.owned.push_back(q);
@@ -66,8 +73,14 @@ static double** eo_work(Ctx& c, int n) {
 //  - while the handle's stream is being captured: a graph that held launches on
 //    the copy would read it as it was at the capture, whatever the fields have
 //    become by its replay.
+// One copy serves a lattice and the handles that borrow its fields, each on a
+// stream of its own and perhaps in a thread of its own: it is made under the
+// lock and complete when the lock is given back, and a call keeps the one it
+// was given.
 template <typename R>
-static const R* eo_compact(Ctx& c) {
+using EoFields = std::shared_ptr<const EoCopy<R>>;
+template <typename R>
+static EoFields<R> eo_compact(Ctx& c) {
   constexpr bool d = std::is_same<R, double>::value;
   const R *U, *C;
   if constexpr (d) {
@@ -83,14 +96,15 @@ static const R* eo_compact(Ctx& c) {
     QWSG_CUDA(cudaStreamIsCapturing(c.st, &cs));
     if (cs != cudaStreamCaptureStatusNone) return nullptr;
   }
-  const Ctx& from = c.parent ? *c.parent : c;
-  const long gen = d ? from.fields_gen_d : from.fields_gen_s;
+  Ctx& owner = eo_owner(c);
+  std::lock_guard<std::mutex> lk(owner.eo_mu);
+  const long gen = d ? owner.fields_gen_d : owner.fields_gen_s;
   const size_t pad = c.eo_pad();
   auto& copy = [&]() -> std::shared_ptr<EoCopy<R>>& {
     if constexpr (d)
-      return c.eoc_d;
+      return owner.eoc_d;
     else
-      return c.eoc_s;
+      return owner.eoc_s;
   }();
   if (!copy) {
     void* q = nullptr;
@@ -103,9 +117,10 @@ static const R* eo_compact(Ctx& c) {
   if (copy->gen != gen) {
     eo_fields<R>(c.G, copy->p, copy->p + 144 * pad, (int)pad, U, C, c.st);
     c.check_launch("eo_fields");
+    QWSG_CUDA(cudaStreamSynchronize(c.st));
     copy->gen = gen;
   }
-  return copy->p;
+  return copy;
 }
 
 // the compact vectors as the BLAS kernels see them: one RHS of Vh sites
@@ -256,9 +271,9 @@ static void solve_mtdagmt(Ctx& c, const double* F, double* out, const double* in
 
 void mtilde_d(Ctx& c, double* out, const double* in) {
   double** v = eo_work(c, 2);
-  if (const double* F = eo_compact<double>(c)) {
+  if (const auto F = eo_compact<double>(c)) {
     eo_gather<double>(c.G, v[1], c.eo_pad(), in, c.pce, c.st);
-    mtilde_c(c, F, v[1], v[1], v[0]);
+    mtilde_c(c, F->p, v[1], v[1], v[0]);
     eo_scatter<double>(c.G, out, v[1], c.eo_pad(), c.pce, false, c.st);
   } else {
     mtilde_p<double>(c, out, in, v[0], -c.kappa * c.kappa);
@@ -269,9 +284,9 @@ void mtilde_d(Ctx& c, double* out, const double* in) {
 
 void mtilde_dag_d(Ctx& c, double* out, const double* in) {
   double** v = eo_work(c, 3);
-  if (const double* F = eo_compact<double>(c)) {
+  if (const auto F = eo_compact<double>(c)) {
     eo_gather<double>(c.G, v[2], c.eo_pad(), in, c.pce, c.st);
-    mtilde_dag_c(c, F, v[2], v[2], v[0], v[1]);
+    mtilde_dag_c(c, F->p, v[2], v[2], v[0], v[1]);
     eo_scatter<double>(c.G, out, v[2], c.eo_pad(), c.pce, false, c.st);
   } else {
     mtilde_dag_p(c, out, in, v[0]);
@@ -283,10 +298,10 @@ void mtilde_s(Ctx& c, float* out, const float* in) {
   eo_work(c, 0);
   float** v = c.eo_s;
   const double coef = -(double)(float)(c.kappa * c.kappa);
-  if (const float* F = eo_compact<float>(c)) {
+  if (const auto F = eo_compact<float>(c)) {
     eo_gather<float>(c.G, v[1], c.eo_pad(), in, c.pce, c.st);
-    eo_apply<float>(c, F, v[0], v[1], c.pco, 0, 1, 0, 0.0, nullptr);
-    eo_apply<float>(c, F, v[1], v[0], c.pce, 0, 1, 2, coef, v[1]);
+    eo_apply<float>(c, F->p, v[0], v[1], c.pco, 0, 1, 0, 0.0, nullptr);
+    eo_apply<float>(c, F->p, v[1], v[0], c.pce, 0, 1, 2, coef, v[1]);
     eo_scatter<float>(c.G, out, v[1], c.eo_pad(), c.pce, false, c.st);
   } else {
     mtilde_p<float>(c, out, in, v[0], coef);
@@ -296,9 +311,9 @@ void mtilde_s(Ctx& c, float* out, const float* in) {
 
 void mtdagmt_d(Ctx& c, double* out, const double* in) {
   double** v = eo_work(c, 4);
-  if (const double* F = eo_compact<double>(c)) {
+  if (const auto F = eo_compact<double>(c)) {
     eo_gather<double>(c.G, v[3], c.eo_pad(), in, c.pce, c.st);
-    mtdagmt_c(c, F, v[3], v[3]);
+    mtdagmt_c(c, F->p, v[3], v[3]);
     eo_scatter<double>(c.G, out, v[3], c.eo_pad(), c.pce, false, c.st);
   } else {
     mtdagmt_p(c, out, in, v[0], v[2]);
@@ -311,7 +326,8 @@ void mtdagmt_d(Ctx& c, double* out, const double* in) {
 // omega step.  x: initial guess in, solution out.  Returns conviter.
 int bicgstab_vm(Ctx& c, double* x, const double* b, int maxiter) {
   double** v = eo_work(c, 9);
-  const double* F = eo_compact<double>(c);
+  const auto fields = eo_compact<double>(c);
+  const double* F = fields ? fields->p : nullptr;
   const Geom G = eo_geom(c);
   double *bb = v[2], *q = v[3], *r = v[4], *p = v[5], *t = v[6], *r0 = v[7], *xx = v[8];
   eo_gather<double>(c.G, bb, G.pad, b, c.pce, c.st);
@@ -359,7 +375,8 @@ static void check_finite(double v, const char* what) {
 // iteration 0 (the reference divides 0 by 0 there).
 int cg_vm(Ctx& c, double* x, const double* b, int maxiter) {
   double** v = eo_work(c, 10);
-  const double* F = eo_compact<double>(c);
+  const auto fields = eo_compact<double>(c);
+  const double* F = fields ? fields->p : nullptr;
   const Geom G = eo_geom(c);
   double *q = v[4], *r = v[5], *p = v[6], *r0 = v[7], *bb = v[8], *xx = v[9];
   eo_gather<double>(c.G, bb, G.pad, b, c.pce, c.st);
@@ -414,7 +431,8 @@ int mcg_vm(Ctx& c, double* X, const double* b, int n, const double* sigma, int m
     c.ms_x = eo_alloc(c, ne * n);
     c.ms_n = n;
   }
-  const double* F = eo_compact<double>(c);
+  const auto fields = eo_compact<double>(c);
+  const double* F = fields ? fields->p : nullptr;
   double *q = v[4], *r = v[5], *p = v[6], *r0 = v[7], *bb = v[8];
   eo_gather<double>(c.G, bb, G.pad, b, c.pce, c.st);
   blas_bicg_init<double>(G, bb, nullptr, r, p, r0, c.d_res, c.rb, c.st);

@@ -396,3 +396,61 @@ def test_without_room_for_a_copy_of_the_fields(bytes_a_site):
                     f(x, out)
                 torch.cuda.synchronize()
         lat.close()
+
+
+def test_borrowing_handles_share_the_copy_of_the_fields():
+    """A one-RHS handle reads its lattice's copy of the fields: its first call
+    takes its work vectors (480 bytes a site and the allocations' rounding),
+    not a copy (1,152) of its own."""
+    L, NB = (16, 16, 16, 32), (2, 1, 1, 1)
+    taken = []
+    for _ in range(2):  # (the first pair loads the kernels)
+        lat = fresh_lattice(L, NB, 3)
+        x = lat.to_device(np.ones((lat.V, 24)))
+        want = lat.mtdagmt(x)
+        child = lat.batch(1)
+        out = child.empty("f64")
+        taken.append(device_memory_of(lambda: child.mtdagmt(x, out=out)))
+        assert np.array_equal(lat.to_host(out), lat.to_host(want))
+        child.close()
+        lat.close()
+    assert taken[1] < 600 * 16 ** 3 * 32 + (4 << 20)
+
+
+def test_threads_share_the_copy_of_the_fields():
+    """A lattice and two handles on its fields, a thread and a stream each, make
+    their first calls after a change of the fields at the same time."""
+    import threading
+
+    import qws_b200
+    import torch
+
+    L, NB = (12, 8, 6, 10), (2, 2, 1, 1)
+    b = qws_b200.gen_source(L, 4)
+    lat = fresh_lattice(L, NB, 1)
+    handles = [lat, lat.batch(1), lat.batch(1)]
+    for h in handles:
+        h.use_own_stream()
+    x, outs = lat.to_device(b), [h.empty("f64") for h in handles]
+    for seed in range(1, 9):
+        lat.gen_gauge_device(seed, 2, 0.36)
+        lat.build_clover(1.0)
+        torch.cuda.synchronize()
+        start = threading.Barrier(len(handles))
+
+        def work(h, out):
+            start.wait()
+            for _ in range(3):
+                h.mtdagmt(x, out=out)
+
+        ts = [threading.Thread(target=work, args=a) for a in zip(handles, outs)]
+        [t.start() for t in ts]
+        [t.join() for t in ts]
+        torch.cuda.synchronize()
+        want = fresh_lattice(L, NB, seed)
+        w = want.mtdagmt(x)
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, w) for o in outs), seed
+        want.close()
+    for h in handles[1:] + [lat]:
+        h.close()
