@@ -224,10 +224,9 @@ struct Ctx {
   static constexpr int kEoVecs = 10, kEoOpVecs = 4;
   double* eo_d[kEoVecs] = {};
   float* eo_s[2] = {};
-  // multi-shift CG: the shifts' search vectors and solutions (ms_n compact
-  // vectors each, back to back)
-  double* ms_p = nullptr;
-  double* ms_x = nullptr;
+  // multi-shift CG: room for ms_n shifts' search vectors and solutions (compact
+  // vectors back to back)
+  double* ms = nullptr;
   int ms_n = 0;
   long n_mtilde = 0;
 

@@ -33,8 +33,9 @@ static cudaError_t eo_try_alloc(void** p, size_t bytes) {
   if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();
   return e;
 }
-// Work vectors come before copies of the fields: where memory holds only one
-// of the two, the copies go (the fields are then read on the full planes).
+// n doubles of work vectors, cleared.  They come before copies of the fields:
+// where memory holds only one of the two, the copies go (the fields are then
+// read on the full planes).
 static double* eo_alloc(Ctx& c, size_t n) {
   void* q = nullptr;
   cudaError_t e = eo_try_alloc(&q, sizeof(double) * n);
@@ -42,8 +43,9 @@ static double* eo_alloc(Ctx& c, size_t n) {
     e = eo_try_alloc(&q, sizeof(double) * n);
   if (e != cudaSuccess)
     throw Error(3, std::string("even-odd work vectors: ") + cudaGetErrorString(e));
-  c.owned.push_back(q);
-  QWSG_CUDA(cudaMemsetAsync(q, 0, sizeof(double) * n, c.st));
+  e = cudaMemsetAsync(q, 0, sizeof(double) * n, c.st);
+  if (e != cudaSuccess) cudaFree(q);
+  QWSG_CUDA(e);
   return static_cast<double*>(q);
 }
 // The first n FP64 work vectors.  Those of the operators (four, and two in
@@ -54,12 +56,14 @@ static double** eo_work(Ctx& c, int n) {
   const size_t ne = (size_t)24 * c.eo_pad();
   if (!c.eo_d[0]) {
     c.eo_d[0] = eo_alloc(c, (Ctx::kEoOpVecs + 1) * ne);
+    c.owned.push_back(c.eo_d[0]);
     for (int i = 1; i < Ctx::kEoOpVecs; i++) c.eo_d[i] = c.eo_d[0] + i * ne;
     c.eo_s[0] = reinterpret_cast<float*>(c.eo_d[0] + Ctx::kEoOpVecs * ne);
     c.eo_s[1] = c.eo_s[0] + ne;
   }
   if (n > Ctx::kEoOpVecs && !c.eo_d[Ctx::kEoOpVecs]) {  // the solvers'
     c.eo_d[Ctx::kEoOpVecs] = eo_alloc(c, (Ctx::kEoVecs - Ctx::kEoOpVecs) * ne);
+    c.owned.push_back(c.eo_d[Ctx::kEoOpVecs]);
     for (int i = Ctx::kEoOpVecs + 1; i < Ctx::kEoVecs; i++)
       c.eo_d[i] = c.eo_d[Ctx::kEoOpVecs] + (i - Ctx::kEoOpVecs) * ne;
   }
@@ -425,12 +429,14 @@ int mcg_vm(Ctx& c, double* X, const double* b, int n, const double* sigma, int m
   const Geom G = eo_geom(c);
   const size_t ne = (size_t)24 * G.pad;
   if (c.ms_n < n) {
-    c.ms_p = c.ms_x = nullptr;  // (the smaller ones stay with the handle)
+    QWSG_CUDA(cudaStreamSynchronize(c.st));
+    cudaFree(c.ms);
+    c.ms = nullptr;
     c.ms_n = 0;
-    c.ms_p = eo_alloc(c, ne * n);
-    c.ms_x = eo_alloc(c, ne * n);
+    c.ms = eo_alloc(c, 2 * ne * n);
     c.ms_n = n;
   }
+  double *ms_p = c.ms, *ms_x = c.ms + ne * n;
   const auto fields = eo_compact<double>(c);
   const double* F = fields ? fields->p : nullptr;
   double *q = v[4], *r = v[5], *p = v[6], *r0 = v[7], *bb = v[8];
@@ -440,8 +446,8 @@ int mcg_vm(Ctx& c, double* X, const double* b, int n, const double* sigma, int m
   const double bnorm = h[0];
   double rho0 = bnorm;
   for (int k = 0; k < n; k++) {
-    blas_zero<double>(G, c.ms_x + k * ne, 0, G.V, c.st);
-    blas_copy<double>(G, c.ms_p + k * ne, r, 0, G.V, c.st);
+    blas_zero<double>(G, ms_x + k * ne, 0, G.V, c.st);
+    blas_copy<double>(G, ms_p + k * ne, r, 0, G.V, c.st);
   }
   if (bnorm == 0) {
     for (int k = 0; k < n; k++)
@@ -473,7 +479,7 @@ int mcg_vm(Ctx& c, double* X, const double* b, int n, const double* sigma, int m
       cf[4 * k + 1] = z2[k];                   // pp_k = z2 r + ...
       cf[4 * k + 2] = beta_new * ratio * ratio;  // ... + beta (z2/z1)^2 pp_k
     }
-    blas_mshift(G, c.ms_x, c.ms_p, n, r, p, beta_new, c.put_coefs(cf.data(), 4 * n), !done, c.st);
+    blas_mshift(G, ms_x, ms_p, n, r, p, beta_new, c.put_coefs(cf.data(), 4 * n), !done, c.st);
     if (done) break;
     beta = beta_new;
     rho0 = rnorm;
@@ -487,7 +493,7 @@ int mcg_vm(Ctx& c, double* X, const double* b, int n, const double* sigma, int m
     alpha0 = alpha;
   }
   for (int k = 0; k < n; k++)
-    eo_scatter<double>(c.G, X + k * c.spinor_elems(), c.ms_x + k * ne, G.pad, c.pce, true, c.st);
+    eo_scatter<double>(c.G, X + k * c.spinor_elems(), ms_x + k * ne, G.pad, c.pce, true, c.st);
   c.check_launch("mcg_vm");
   return iter;
 }

@@ -219,6 +219,7 @@ const double* Ctx::put_coefs(const double* v, int n) {
 Ctx::~Ctx() {
   if (st) cudaStreamSynchronize(st);
   for (void* p : owned) cudaFree(p);
+  cudaFree(ms);
   if (stage) cudaFree(stage);
   for (cudaEvent_t e : ev_pool) cudaEventDestroy(e);
   clear_graphs();

@@ -454,3 +454,42 @@ def test_threads_share_the_copy_of_the_fields():
         want.close()
     for h in handles[1:] + [lat]:
         h.close()
+
+
+def test_shift_vectors_are_given_back():
+    """mcg_vm's vectors: an outgrown block goes back, and a call for which there
+    is no room takes nothing."""
+    import qws_b200
+    import torch
+
+    L, NB = (16, 16, 16, 16), (2, 1, 1, 1)
+    lat = fresh_lattice(L, NB, 3)
+    X = torch.zeros(32 * 24 * lat.pad, dtype=torch.float64, device="cuda")
+    bd = lat.to_device(qws_b200.gen_source(L, 4))
+
+    def mcg(n):  # two iterations, into X
+        import ctypes
+
+        sigma, it = np.linspace(0.0, 1.0, n), ctypes.c_int()
+        return lat.lib.qwsg_mcg_vm(lat.h, X.data_ptr(), bd.data_ptr(), n,
+                                   ctypes.c_void_p(sigma.ctypes.data), 3, ctypes.byref(it))
+
+    one_shift = 2 * 96 * lat.V
+    assert mcg(2) == 0
+    grown = device_memory_of(lambda: [mcg(n) for n in (3, 4, 6, 8)])
+    assert grown < 6 * one_shift + (4 << 20)
+    torch.cuda.empty_cache()
+    fill, chunk, keep = [], 2 << 20, 14 * one_shift
+    while (free := torch.cuda.mem_get_info()[0]) > keep + chunk:
+        fill.append(torch.empty((free - keep) // chunk * chunk, dtype=torch.uint8, device="cuda"))
+    try:
+        # 32 shifts do not fit, not even with the block of eight and the copy of
+        # the fields (6 shifts' worth) given back for them
+        rc = []
+        taken = device_memory_of(lambda: rc.extend(mcg(32) for _ in range(3)))
+    finally:
+        fill.clear()
+        torch.cuda.empty_cache()
+    assert 0 not in rc and taken < 0
+    assert mcg(32) == 0
+    lat.close()
