@@ -149,6 +149,7 @@ struct Ctx {
   // per-RHS statistics of the last multi-RHS solve
   std::vector<SolveStats> last_stats;
   std::vector<int> last_iters;
+  void* device_alloc(size_t bytes);
   template <typename R>
   R* alloc_spinor();
   void ensure_sap();

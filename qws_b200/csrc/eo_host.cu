@@ -17,33 +17,10 @@ namespace qwsg {
   throw Error(2, "even-odd operator: unsupported combination of hop set / adjoint / clover / mode");
 }
 
-// whose copy of the fields a handle reads: that of the lattice they live on
-static Ctx& eo_owner(Ctx& c) { return c.parent ? *c.parent : c; }
-
-bool Ctx::release_copies() {
-  std::lock_guard<std::mutex> lk(eo_mu);
-  if (!eoc_d && !eoc_s) return false;
-  eoc_d.reset();
-  eoc_s.reset();
-  return true;
-}
-
-static cudaError_t eo_try_alloc(void** p, size_t bytes) {
-  const cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();
-  return e;
-}
-// n doubles of work vectors, cleared.  They come before copies of the fields:
-// where memory holds only one of the two, the copies go (the fields are then
-// read on the full planes).
+// n doubles of work vectors, cleared
 static double* eo_alloc(Ctx& c, size_t n) {
-  void* q = nullptr;
-  cudaError_t e = eo_try_alloc(&q, sizeof(double) * n);
-  if (e == cudaErrorMemoryAllocation && eo_owner(c).release_copies())
-    e = eo_try_alloc(&q, sizeof(double) * n);
-  if (e != cudaSuccess)
-    throw Error(3, std::string("even-odd work vectors: ") + cudaGetErrorString(e));
-  e = cudaMemsetAsync(q, 0, sizeof(double) * n, c.st);
+  void* q = c.device_alloc(sizeof(double) * n);
+  const cudaError_t e = cudaMemsetAsync(q, 0, sizeof(double) * n, c.st);
   if (e != cudaSuccess) cudaFree(q);
   QWSG_CUDA(e);
   return static_cast<double*>(q);
@@ -100,7 +77,7 @@ static EoFields<R> eo_compact(Ctx& c) {
     QWSG_CUDA(cudaStreamIsCapturing(c.st, &cs));
     if (cs != cudaStreamCaptureStatusNone) return nullptr;
   }
-  Ctx& owner = eo_owner(c);
+  Ctx& owner = c.parent ? *c.parent : c;
   std::lock_guard<std::mutex> lk(owner.eo_mu);
   const long gen = d ? owner.fields_gen_d : owner.fields_gen_s;
   const size_t pad = c.eo_pad();
@@ -112,8 +89,11 @@ static EoFields<R> eo_compact(Ctx& c) {
   }();
   if (!copy) {
     void* q = nullptr;
-    const cudaError_t e = eo_try_alloc(&q, sizeof(R) * 288 * pad);
-    if (e == cudaErrorMemoryAllocation) return nullptr;
+    const cudaError_t e = cudaMalloc(&q, sizeof(R) * 288 * pad);
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
     if (e != cudaSuccess)
       throw Error(3, std::string("even-odd copy of the fields: ") + cudaGetErrorString(e));
     copy = std::make_shared<EoCopy<R>>(static_cast<R*>(q));

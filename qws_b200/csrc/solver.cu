@@ -244,10 +244,34 @@ Ctx::~Ctx() {
   if (own_stream && st) cudaStreamDestroy(st);
 }
 
+bool Ctx::release_copies() {
+  std::lock_guard<std::mutex> lk(eo_mu);
+  if (!eoc_d && !eoc_s) return false;
+  eoc_d.reset();
+  eoc_s.reset();
+  return true;
+}
+
+// Device memory for work buffers.  They come before the compact copies of the
+// fields: where memory holds only one of the two, the copies go (the even-odd
+// operators then read the fields on the full planes).
+void* Ctx::device_alloc(size_t bytes) {
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    if ((parent ? parent : this)->release_copies()) {
+      e = cudaMalloc(&p, bytes);
+      if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();
+    }
+  }
+  if (e != cudaSuccess) throw Error(3, std::string("work buffers: ") + cudaGetErrorString(e));
+  return p;
+}
+
 template <typename R>
 R* Ctx::alloc_spinor() {
-  R* p = nullptr;
-  QWSG_CUDA(cudaMalloc(&p, sizeof(R) * spinor_elems()));
+  R* p = static_cast<R*>(device_alloc(sizeof(R) * spinor_elems()));
   QWSG_CUDA(cudaMemsetAsync(p, 0, sizeof(R) * spinor_elems(), st));
   owned.push_back(p);
   return p;
@@ -257,9 +281,8 @@ template double* Ctx::alloc_spinor<double>();
 
 // FP16 spinor: three 16-byte planes + one float plane of per-site scales (IO<H16>)
 __half* Ctx::alloc_spinor_h() {
-  void* p = nullptr;
   const size_t bytes = (size_t)(6 * 8 + 4) * spad(G);
-  QWSG_CUDA(cudaMalloc(&p, bytes));
+  void* p = device_alloc(bytes);
   QWSG_CUDA(cudaMemsetAsync(p, 0, bytes, st));
   owned.push_back(p);
   return (__half*)p;

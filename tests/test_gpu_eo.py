@@ -493,3 +493,39 @@ def test_shift_vectors_are_given_back():
     assert 0 not in rc and taken < 0
     assert mcg(32) == 0
     lat.close()
+
+
+def test_copies_give_way_to_other_work_buffers():
+    """After an even-odd operator, with 1,400 bytes of device memory a site left,
+    a DD solve whose buffers need 2,208 takes those of the copy of the fields
+    (1,152), and the operator still runs."""
+    import qws_b200
+    import torch
+
+    L, NB = (16, 16, 16, 32), (2, 1, 1, 1)
+    res = []
+    for scarce in (False, True):  # (the first handle loads the kernels)
+        lat = fresh_lattice(L, NB, 3)
+        bd = lat.to_device(qws_b200.gen_source(L, 4))
+        x, out, again = (torch.zeros_like(bd) for _ in range(3))
+        lat.mtdagmt(bd, out=out)
+        lat.deo(bd, 0, clov=1, out=again)
+        lat.ddd(bd, out=again)
+        lat.ddd(bd.float())
+        again.zero_()
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        fill, chunk, keep = [], 2 << 20, 1400 * lat.V
+        while scarce and (free := torch.cuda.mem_get_info()[0]) > keep + chunk:
+            fill.append(torch.empty((free - keep) // chunk * chunk, dtype=torch.uint8, device="cuda"))
+        try:
+            lat.bicgstab_dd_mix(x, bd, 1e-10, 20, 1e-6, 50)
+            lat.mtdagmt(bd, out=again)
+            torch.cuda.synchronize()
+        finally:
+            fill.clear()
+            torch.cuda.empty_cache()
+        assert close(again, out)
+        res.append(x)
+        lat.close()
+    assert torch.equal(*res)
