@@ -81,6 +81,24 @@ double hop_bytes(int sel, int epi, int nr, bool links12 = false) {
   return 2 * sp + lc;                       // in, out
 }
 
+// what the SAP update with all hops reads of the other colour, per site it
+// handles: the spinors of the sites a face hop reaches (two spins of those it
+// reaches over one face in t alone) and the links of its backward face hops.
+// (Where the block grid has extent 1 the neighbour across the face is the
+// block itself, which hop_bytes counts.)
+template <typename T>
+double update_face_bytes(const Geom& G, bool links12) {
+  double apart = 1, links = 0;  // sites no face hop in x, y or z reaches
+  for (int mu = 0; mu < 4; mu++) {
+    if (G.NB[mu] == 1) continue;
+    if (mu < 3) apart *= G.B[mu] > 2 ? 1.0 - 2.0 / G.B[mu] : 0.0;
+    links += Bytes<T>::links / 4.0 / G.B[mu];
+  }
+  double spinors = 1 - apart;
+  if (G.NB[3] > 1) spinors += apart * (G.B[3] == 1 ? 1.0 : 0.5 * 2.0 / G.B[3]);
+  return spinors * Bytes<T>::spinor * G.nr + links * (links12 ? 2.0 / 3 : 1.0);
+}
+
 template <typename T>
 int kind_of(int sel, int epi) {
   const bool d = sizeof(typename Store<T>::type) == 8;
@@ -114,10 +132,8 @@ void run_hop(Ctx& c, int sel, int epi, const HopArgs<T>& a) {
   if (sel == HOP_OUTER && !a.list) sites = face_sites_per_colour(c.G) * (a.nsites == c.G.V ? 2 : 1);
   if (a.dom >= 0) sites /= 2;
   double bytes = (double)sites * hop_bytes<T>(sel, epi, c.G.nr, a.U12 != nullptr);
-  if (sel == HOP_ALL && epi == EPI_SAPE)  // the other colour's sites next to the faces, and
-    for (int mu = 0; mu < 4; mu++)        // the links of the backward half of those hops
-      bytes += 2.0 * a.nsites / c.G.B[mu] *
-               (Bytes<T>::spinor * c.G.nr / (mu == 3 ? 2 : 1) + Bytes<T>::links / 8);
+  if (sel == HOP_ALL && epi == EPI_SAPE)
+    bytes += a.nsites * update_face_bytes<T>(c.G, a.U12 != nullptr);
   c.recs.push_back({kind_of<T>(sel, epi), e0, e1, bytes});
 }
 
