@@ -59,10 +59,11 @@ def test_shipped_cache_is_valid():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("threads", [64, 256])
-def test_hop_threads_bit_equal(threads):
+@pytest.mark.parametrize("L", [(8, 8, 8, 16),       # FP32 and FP16 in k_hop_split, whose CTA is fixed
+                               (18, 18, 22, 20)])   # above its sizes, the last CTA not full
+def test_hop_threads_bit_equal(threads, L):
     import qws_b200
 
-    L = (8, 8, 8, 16)
     U, _ = qws_b200.gen_gauge(L, 7, 5, 0.36)
     C = qws_b200.gen_clover(U, L, 1.7, 0.1365)
     lat = qws_b200.Lattice(L, (2, 2, 2, 2), tbc=-1, kappa=0.1365)

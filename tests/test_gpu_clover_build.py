@@ -122,3 +122,40 @@ def test_clover_operator_at_edges(shape, NB, csw):
     finally:
         host.close()
         dev.close()
+
+
+def test_batch_with_some_indefinite_blocks():
+    """A kappa per right-hand side, of which one gives indefinite clover blocks
+    (the pivoted inverse, at that right-hand side's entries alone): the FP64 and
+    FP32 operators and the FP16 SAP of every right-hand side against those of a
+    lattice with that kappa.  Both sides make the same clover term, bit for bit,
+    and run the same sums, so FP64 and FP32 differ by at most a rounding of the
+    result (2^-53, 2^-24 relative) and the SAP by that of its FP16 storage in
+    each of its sweeps (2^-11, four times)."""
+    import qws_b200
+
+    shape, NB, csw = (4, 4, 6, 8), (2, 1, 1, 1), 12.0
+    kappas = [0.002, KAPPA, 0.001, 0.003]
+    U, _ = qws_b200.gen_gauge(shape, 8, 5, 0.36)
+    lat = qws_b200.Lattice(shape, NB, tbc=-1, kappa=0.002)
+    many = None
+    try:
+        lat.load_gauge(U)
+        lat.build_clover(csw)
+        many = lat.batch(4)
+        many.set_kappas(kappas, csw)
+        x = np.stack([qws_b200.gen_source(shape, 9 + r) for r in range(4)])
+        xd, xs = many.to_device(x), many.to_device(x.astype(np.float32))
+        got = {"ddd": many.to_host(many.ddd(xd)), "ddd_s": many.to_host(many.ddd(xs)),
+               "prec_h": many.to_host(many.prec_h(xs, 2, 2))}
+        for r, k in enumerate(kappas):
+            lat.set_kappa(k)
+            lat.build_clover(csw)
+            one, ones = lat.to_device(x[r]), lat.to_device(x[r].astype(np.float32))
+            assert rel(got["ddd"][r], lat.to_host(lat.ddd(one))) < 2**-53, k
+            assert rel(got["ddd_s"][r], lat.to_host(lat.ddd(ones))) < 2**-24, k
+            assert rel(got["prec_h"][r], lat.to_host(lat.prec_h(ones, 2, 2))) < 4 * 2**-11, k
+    finally:
+        if many:
+            many.close()
+        lat.close()

@@ -21,6 +21,11 @@ pytestmark = pytest.mark.gpu
 CSW, KAPPA = 1.7, 0.1365
 
 
+# small enough for k_hop_split in FP32 and FP16, and with every launch above
+# that size (the face lists of 42,904 sites too), the last 128 sites not filled
+SMALL_AND_LARGE = [((8, 8, 8, 16), (2, 2, 2, 2)), ((18, 18, 22, 20), (2, 2, 2, 2))]
+
+
 def lattice(L, NB, seed):
     import qws_b200
 
@@ -30,11 +35,11 @@ def lattice(L, NB, seed):
     return lat
 
 
-def test_solves_reproducible_across_runs_graphs_and_cta_sizes():
+@pytest.mark.parametrize("L, NB", SMALL_AND_LARGE)
+def test_solves_reproducible_across_runs_graphs_and_cta_sizes(L, NB):
     import qws_b200
     import torch
 
-    L, NB = (8, 8, 8, 16), (2, 2, 2, 2)
     lat = lattice(L, NB, 21)
     bd = lat.to_device(qws_b200.gen_source(L, 22))
 
@@ -80,11 +85,12 @@ def padding(x, lat):
     return x.view(12, lat.pad, 2)[:, lat.V:, :]
 
 
-def test_padding_canaries():
+@pytest.mark.parametrize("L, NB", [((12, 6, 4, 6), (2, 1, 1, 1)),  # 1728 sites, planes of 1792
+                                   SMALL_AND_LARGE[1]])
+def test_padding_canaries(L, NB):
     import qws_b200
     import torch
 
-    L, NB = (12, 6, 4, 6), (2, 1, 1, 1)   # 1728 sites, planes of 1792
     lat = lattice(L, NB, 31)
     assert lat.pad > lat.V
     b = qws_b200.gen_source(L, 32)

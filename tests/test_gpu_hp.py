@@ -179,3 +179,38 @@ def test_graphs_updated_for_a_new_kappa_match_direct_launches():
     np.testing.assert_array_equal(xg, xd)
     assert sg["inner_iters"] == sd["inner_iters"] and sg["outer_iters"] == sd["outer_iters"]
     assert tg < 1e-10
+
+
+@pytest.mark.parametrize("L, NB", [((8, 8, 8, 8), (2, 2, 2, 2)), ((12, 12, 12, 24), (2, 1, 1, 1))])
+def test_merged_update_no_further_from_fp32_than_two_passes(L, NB):
+    """The SAP updates s by its block and by the faces in one pass and stores it
+    once; as two passes (the block update, then the face hops, each stored in
+    FP16) the same sweeps are the reference's sequence.  Against the FP32 SAP,
+    whose own rounding is a thousand times smaller, the merged form must be no
+    further off: it has one FP16 rounding of s fewer in every half-sweep."""
+    import qws_b200
+
+    nsap, nm, k = 4, 3, 0.1365
+    lat = qws_b200.Lattice(L, NB, tbc=-1, kappa=k)
+    try:
+        lat.gen_gauge_device(3, 5, 0.36)
+        lat.build_clover(1.7)
+        for seed in (1, 2, 3):
+            b = lat.store_h(lat.to_device(qws_b200.gen_source(L, seed).astype(np.float32)))
+            s, a = b.clone(), b.new_zeros(b.shape)
+            for _ in range(nsap - 1):
+                for e in (0, 1):
+                    lat.jinv_h(s, e, nm, out=a)
+                    lat.sap_update(s, a, b, e, half=True)
+                    lat.ddd_out_h(a, 1 - e, k, out=s)
+            two, x0 = b.new_zeros(b.shape), b.new_zeros(b.shape)
+            lat.jinv_h(s, 0, nm, out=x0)
+            lat.ddd_out_h(x0, 1, k, out=s)
+            lat.jinv_h(s, 0, nm, out=two)
+            lat.jinv_h(s, 1, nm, out=two)
+            want = lat.prec(b, nsap - 1, nm).double()
+            off = lambda x: float((x.double() - want).norm() / want.norm())
+            one = lat.prec_h(b, nsap, nm)
+            assert off(one) < off(two) < 1e-3, (off(one), off(two))
+    finally:
+        lat.close()
