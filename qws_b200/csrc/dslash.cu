@@ -571,8 +571,11 @@ __global__ void __launch_bounds__(128) k_hop_split(const HopArgs<T> a) {
 
 // Several lattices in one launch (a group solve; one right-hand side each):
 // block b runs threads [(b - starts[l]) * blockDim, ...) of member l's own
-// launch, with l's arguments copied into shared memory first, so every
-// member runs exactly the code and arithmetic of its own launch.
+// launch, with l's arguments copied into shared memory first.  Every member's
+// result is bit for bit that of its own launch: the same body, or, where its
+// own launch is small enough for k_hop_split, that kernel's sums in the same
+// order (a group's launch is large where its members' are small, so here one
+// thread takes a site).
 template <typename T, int SEL, int EPI>
 __device__ __forceinline__ void hop_multi_body(const HopArgs<T>* __restrict__ args,
                                                const int* __restrict__ starts, int n) {
@@ -621,6 +624,9 @@ static void launch_v(const HopArgs<T>& a, cudaStream_t st) {
       return;
     }
   }
+  // (the FP32 update with all hops and a kappa per RHS lands in k_hop, at 104
+  // registers; M_SAP with four kappas 5.28 -> 5.15 ms at 24^3x48 and 1.22 ->
+  // 1.15 at 16^3x32 against the bounded update and face passes it replaces)
   if constexpr (MinCtas<T, SEL>::value == 4)
     k_hop_r64<T, SEL, EPI, PRK><<<blocks, threads, 0, st>>>(a);
   else
@@ -641,7 +647,11 @@ static void launch(const HopArgs<T>& a, cudaStream_t st) {
 // work does not depend on the CTA size), each member's sites in its own
 // blocks; the FP16 block kernels keep their 64-register bound (the FP32
 // block kernels and the full-lattice operators would spill under the bounds
-// of their one-lattice forms, where the arguments sit in kernel parameters)
+// of their one-lattice forms, where the arguments sit in kernel parameters).
+// The FP16 update with all hops is unbounded, at 101 registers; beside the
+// update at 64 and the face pass at 80 that it replaces, the group's time on
+// the GPU fell: 38.3 -> 35.4 ms for 48 lattices of 8^4 and 12^3x24, 28.0 -> 26.7
+// for eight of 16^3x32, 69.4 -> 68.1 for four of 24^3x48.
 template <typename T, int SEL, int EPI>
 static void merge_hop(const GroupRec* const* recs, int n, GroupBatch& b) {
   constexpr int threads = 128;
