@@ -185,6 +185,8 @@ def run_reference(w, warmup, steps, solution_out=None, threads=None):
     env["CUDA_VISIBLE_DEVICES"] = ""
     res = subprocess.run([sys.executable, str(ROOT / "oracle" / "refbench.py"), json.dumps(spec)],
                          capture_output=True, text=True, env=env, timeout=3600)
+    if res.returncode == 3:  # refbench.NOT_BUILT
+        raise FileNotFoundError(res.stderr.strip())
     if res.returncode != 0:
         raise RuntimeError("reference run failed: " + res.stderr[-2000:])
     return json.loads(res.stdout.strip().splitlines()[-1])
@@ -1152,7 +1154,11 @@ def bench_reference(args, w, name):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
-    ref = run_reference(w, args.warmup, args.steps)
+    try:
+        ref = run_reference(w, args.warmup, args.steps)
+    except FileNotFoundError as e:
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        return
     v = ref["solves_per_s"]
     line = {
         "impl": "reference",

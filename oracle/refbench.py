@@ -77,6 +77,10 @@ def read_counts(path):
     return out
 
 
+#: exit status where the reference's library does not exist
+NOT_BUILT = 3
+
+
 def main():
     spec = json.loads(sys.argv[1])
     import qwsref
@@ -84,6 +88,10 @@ def main():
 
     L = tuple(spec["L"])
     variant = spec.get("variant") or pick_variant(L)
+    if not qwsref.ref_variant_path(variant).exists():
+        sys.stderr.write(f"the reference's library for this lattice ({variant}) is not built here: "
+                         "its sources were not present\n")
+        sys.exit(NOT_BUILT)
     t0 = time.time()
     U, plaq = qwsref.gen_gauge(L, spec["seed"], spec["n_smear"], spec["alpha"])
     C = qwsref.gen_clover(U, L, spec["csw"], spec["kappa"])

@@ -34,3 +34,25 @@ def test_kernel_table():
     assert row["GFLOPs"] == pytest.approx(1872 * Vh / 1e-3 / 1e9, rel=1e-3)
     # without the geometry the table has no GFLOP/s
     assert "GFLOPs" not in bench.kernel_table({"jinv_step_f32": (1, 1.0, 1.0)}, 1.0)["jinv_step_f32"]
+
+
+def test_reference_arm_without_its_library(tmp_path):
+    """Where the reference's library was not built, the arm says so in one JSON
+    line and exits 0."""
+    import json
+    import os
+    import shutil
+    import subprocess
+
+    root = Path(bench.__file__).resolve().parent
+    (tmp_path / "oracle").mkdir()
+    shutil.copy(root / "bench.py", tmp_path)
+    for f in ("refbench.py", "qwsref.py", "liboracle.so"):
+        if (root / "oracle" / f).exists():
+            shutil.copy(root / "oracle" / f, tmp_path / "oracle")
+    env = dict(os.environ, PYTHONPATH=str(root))
+    res = subprocess.run([sys.executable, str(tmp_path / "bench.py"), "--impl", "reference"],
+                         capture_output=True, text=True, env=env, timeout=300)
+    assert res.returncode == 0, res.stderr
+    line = json.loads(res.stdout.strip().splitlines()[-1])
+    assert line["impl"] == "reference" and "not built" in line["unavailable"]
