@@ -279,7 +279,12 @@ int qwsg_gen_source(double* S, const int L[4], unsigned long long seed, int kind
  *   mode  0 out = hops, 1 out += factor*hops, 2 out = in0 + factor*hops
  *         (one_minus_*).
  * deo and clv take no device memory of their own (capturable from the first
- * call on). */
+ * call on).  mtilde, mtilde_dag and mtdagmt take 480 bytes a site on the first
+ * use of any of them (capturable after it) and, where there is room, keep a
+ * re-ordered copy of the fields: 1,152 bytes a site in FP64, 576 in FP32, one
+ * for a lattice and the one-RHS handles on it, given back when another buffer
+ * of theirs needs the room.  The solvers take 576 bytes a site more, mcg_vm
+ * 192 for each shift besides. */
 int qwsg_set_parities(qwsg_lattice* lat, int pce, int pco);
 int qwsg_deo_d(qwsg_lattice* lat, double* out, const double* in, int pe, int which, int dag,
                int clov, int mode, double factor, const double* in0);

@@ -231,7 +231,7 @@ struct Ctx {
   int ms_n = 0;
   long n_mtilde = 0;
 
-  // CUDA graphs of the SAP preconditioner's launch sequences (about 40
+  // CUDA graphs of the SAP preconditioner's launch sequences (about 30
   // launches, no host synchronisation inside), captured on first use per
   // (operator, buffers, nsap, nm, kappa) and replayed afterwards.  Off while
   // kernel timing is on and on the legacy default stream.

@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(256) k_hop_pair(const HopArgs<H16> a) {
 // Most sites of such a launch.  Measured per SAP application (one thread ->
 // four threads a site): FP32 at 2,048 sites a launch 188 -> 98 us, 20,736:
 // 224 -> 173, 27,440: 242 -> 213, 38,416: 265 -> 281 (D alone at 30,240 sites
-// 10.2 -> 8.2, at 38,416 10.4 -> 12.2); FP16 (more instructions
+// 10.2 -> 9.0, at 38,416 10.4 -> 12.2); FP16 (more instructions
 // a site, so an SM fills earlier) 150 -> 102, 190 -> 172, 198 -> 207,
 // 222 -> 268.
 template <typename T>

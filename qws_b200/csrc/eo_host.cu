@@ -1,8 +1,10 @@
 // Host side of the even-odd (site parity) operator family and its solver
 // (deo_*/dee_*/one_minus_*, clvd_vm_/clv_s_, mtilde_vm_, mtilde_dag_vm_,
 // mtilde_s_ of qws.cc:390-605 and bicgstab_vm_ of bicgstab.cc:68-333).
-// At the API a parity-p vector is the parity-p sites of full DD-order planes;
-// the operators and solvers here run on compact one-parity vectors (eo.cu).
+// At the API a parity-p vector is the parity-p sites of full DD-order planes.
+// Single operators run on those; the Schur operators and solvers run on compact
+// one-parity vectors, and on a compact copy of the fields where there can be one
+// (eo.cu).
 #include <cmath>
 #include <complex>
 #include <string>
