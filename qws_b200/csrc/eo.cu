@@ -30,23 +30,6 @@
 
 namespace qwsg {
 
-// compact index of the site with coordinates x, within its parity
-__device__ __forceinline__ int eo_index(const Geom& G, const int x[4]) {
-  return (x[0] >> 1) + (G.L[0] >> 1) * (x[1] + G.L[1] * (x[2] + G.L[2] * x[3]));
-}
-
-// coordinates of entry e of parity p
-__device__ __forceinline__ void eo_coords(const Geom& G, int e, int p, int x[4]) {
-  const int nxh = G.L[0] >> 1;
-  int k = e / nxh;
-  const int xh = e - k * nxh;
-  x[1] = k % G.L[1];
-  k /= G.L[1];
-  x[3] = k / G.L[2];
-  x[2] = k - x[3] * G.L[2];
-  x[0] = 2 * xh + ((p + x[1] + x[2] + x[3]) & 1);
-}
-
 struct EoSite {
   int xh, y, z, t;
   int odd;  // x = 2 xh + odd
@@ -86,19 +69,8 @@ __device__ __forceinline__ void eo_hop_with(const R u[18], const R v[24], bool t
 
 template <typename T, int DAG, int MU, int DIR, typename R = typename Arith<T>::R>
 __device__ __forceinline__ void eo_hop(const EoArgs<T>& a, const EoSite& s, int e, R acc[24]) {
-  const int nxh = a.G.L[0] >> 1;
-  const int c = MU == 0 ? 2 * s.xh + s.odd : MU == 1 ? s.y : MU == 2 ? s.z : s.t;
-  int en = e;
-  if (MU == 0) {
-    // x+1 of an even x and x-1 of an odd x have the same compressed index
-    if (DIR > 0 && s.odd) en = s.xh + 1 == nxh ? e - (nxh - 1) : e + 1;
-    if (DIR < 0 && !s.odd) en = s.xh == 0 ? e + (nxh - 1) : e - 1;
-  } else {
-    const int str = MU == 1 ? nxh : MU == 2 ? nxh * a.G.L[1] : nxh * a.G.L[1] * a.G.L[2];
-    const int L = a.G.L[MU];
-    en = DIR > 0 ? (c + 1 == L ? e - (L - 1) * str : e + str)
-                 : (c == 0 ? e + (L - 1) * str : e - str);
-  }
+  const int c = MU == 0 ? 0 : MU == 1 ? s.y : MU == 2 ? s.z : s.t;
+  const int en = eo_step(a.G, e, MU, DIR, c, s.xh, s.odd);
   R v[24], u[18];
   if (MU == 3)
     IO<T>::load_half(a.src, a.pad, en, (DAG ? -DIR : DIR) > 0, v);
@@ -150,15 +122,13 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) k_eo(const EoArgs
 // at 8^3x16 10 us (19 / 21; 17).
 template <typename T, int WHICH, int DAG, int MU, int DIR, typename R = typename Arith<T>::R>
 __device__ __forceinline__ void eo_hop_planes(const EoArgs<T>& a, const int x[4], int g, R acc[24]) {
-  const int L = a.G.L[MU];
   if (WHICH != 3) {
     const int box = a.box[MU], in_box = x[MU] % box;
     const bool inner = DIR > 0 ? in_box != box - 1 : in_box != 0;
     if (inner ? !(WHICH & 1) : !(WHICH & 2)) return;
   }
-  int xn[4] = {x[0], x[1], x[2], x[3]};
-  xn[MU] = DIR > 0 ? (x[MU] + 1 == L ? 0 : x[MU] + 1) : (x[MU] == 0 ? L - 1 : x[MU] - 1);
-  if (MU > 0) xn[0] = 2 * (x[0] >> 1) + ((1 - a.pe + xn[1] + xn[2] + xn[3]) & 1);
+  int xn[4];
+  eo_neighbour<MU, DIR>(a.G, x, a.pe, xn);
   const int gn = dd_index(a.G, xn);
   R v[24], u[18];
   if (MU == 3)
@@ -166,7 +136,7 @@ __device__ __forceinline__ void eo_hop_planes(const EoArgs<T>& a, const int x[4]
   else
     IO<T>::load_spinor(a.src, a.G.pad, gn, v);
   IO<T>::load_link(a.U[0], a.G.pad, MU, DIR > 0 ? g : gn, u);
-  eo_hop_with<T, DAG, MU, DIR>(u, v, DIR > 0 ? x[3] == L - 1 : x[3] == 0, a.G.tbc, acc);
+  eo_hop_with<T, DAG, MU, DIR>(u, v, DIR > 0 ? x[3] == a.G.L[3] - 1 : x[3] == 0, a.G.tbc, acc);
 }
 template <typename T, int WHICH, int DAG, int CLOV, int MODE>
 __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) k_eo_planes(const EoArgs<T> a) {
@@ -176,16 +146,10 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) k_eo_planes(const
   int x[4], x1[4];
   site_coords(a.G, 2 * i, x);
   site_coords(a.G, 2 * i + 1, x1);
-  const bool first = ((x[0] + x[1] + x[2] + x[3]) & 1) == a.pe;
-  bool second = ((x1[0] + x1[1] + x1[2] + x1[3]) & 1) == a.pe;
-  if (!first && !second) return;
-  int g = 2 * i;
-  if (!first) {
-    g++;
-#pragma unroll
-    for (int k = 0; k < 4; k++) x[k] = x1[k];
-    second = false;
-  }
+  bool second;
+  int g = eo_first(x, x1, a.pe, second);
+  if (g < 0) return;
+  g += 2 * i;
   for (;;) {
     R acc[24];
 #pragma unroll

@@ -217,11 +217,69 @@ __host__ __device__ __forceinline__ int dd_index(const Geom& G, const int x[4]) 
 }
 
 // global coordinates of the site with DD-order index g
-__device__ __forceinline__ void site_coords(const Geom& G, int g, int x[4]) {
+__host__ __device__ __forceinline__ void site_coords(const Geom& G, int g, int x[4]) {
   Site s;
   decode_site(G, g, s);
 #pragma unroll
   for (int mu = 0; mu < 4; mu++) x[mu] = s.bc[mu] * G.B[mu] + s.lc[mu];
+}
+
+// Site parity (even-odd operators, eo.cu).  Compact index of the site with
+// coordinates x, within its parity
+__host__ __device__ __forceinline__ int eo_index(const Geom& G, const int x[4]) {
+  return (x[0] >> 1) + (G.L[0] >> 1) * (x[1] + G.L[1] * (x[2] + G.L[2] * x[3]));
+}
+// coordinates of entry e of parity p
+__host__ __device__ __forceinline__ void eo_coords(const Geom& G, int e, int p, int x[4]) {
+  const int nxh = G.L[0] >> 1;
+  int k = e / nxh;
+  const int xh = e - k * nxh;
+  x[1] = k % G.L[1];
+  k /= G.L[1];
+  x[3] = k / G.L[2];
+  x[2] = k - x[3] * G.L[2];
+  x[0] = 2 * xh + ((p + x[1] + x[2] + x[3]) & 1);
+}
+// the site of the other parity that a hop of parity p's site x reads: a y/z/t
+// hop keeps the compressed index x/2, also across a boundary
+template <int MU, int DIR>
+__host__ __device__ __forceinline__ void eo_neighbour(const Geom& G, const int x[4], int p,
+                                                      int xn[4]) {
+  const int L = G.L[MU];
+#pragma unroll
+  for (int k = 0; k < 4; k++) xn[k] = x[k];
+  xn[MU] = DIR > 0 ? (x[MU] + 1 == L ? 0 : x[MU] + 1) : (x[MU] == 0 ? L - 1 : x[MU] - 1);
+  if (MU > 0) xn[0] = 2 * (x[0] >> 1) + ((1 - p + xn[1] + xn[2] + xn[3]) & 1);
+}
+// its compact index, from entry e of parity p: c the coordinate along mu, xh =
+// x/2, odd = x & 1
+__host__ __device__ __forceinline__ int eo_step(const Geom& G, int e, int mu, int dir, int c, int xh,
+                                                int odd) {
+  const int nxh = G.L[0] >> 1;
+  if (mu == 0) {
+    // x+1 of an even x and x-1 of an odd x have the same compressed index
+    if (dir > 0 && odd) return xh + 1 == nxh ? e - (nxh - 1) : e + 1;
+    if (dir < 0 && !odd) return xh == 0 ? e + (nxh - 1) : e - 1;
+    return e;
+  }
+  const int str = mu == 1 ? nxh : mu == 2 ? nxh * G.L[1] : nxh * G.L[1] * G.L[2];
+  const int L = G.L[mu];
+  return dir > 0 ? (c + 1 == L ? e - (L - 1) * str : e + str)
+                 : (c == 0 ? e + (L - 1) * str : e - str);
+}
+// the sites of parity p among 2i and 2i + 1 of the planes' order: x the
+// coordinates of 2i and x1 of 2i + 1 on entry, x those of the first such site
+// (2i + its return value; -1: none) on return, `second` if 2i + 1 is another
+__host__ __device__ __forceinline__ int eo_first(int (&x)[4], const int (&x1)[4], int p,
+                                                 bool& second) {
+  const bool first = ((x[0] + x[1] + x[2] + x[3]) & 1) == p;
+  second = ((x1[0] + x1[1] + x1[2] + x1[3]) & 1) == p;
+  if (!first && !second) return -1;
+  if (first) return 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) x[k] = x1[k];
+  second = false;
+  return 1;
 }
 
 // index of the neighbour across the block face in direction mu (dir = +1/-1)

@@ -3,7 +3,8 @@ index functions of qws_b200/csrc/lattice.cuh are __host__ __device__, so
 tests/geometry_check.cu (built here with nvcc, run without a GPU) drives the
 exact device code -- the DD-order bijection, the in-block hops with the
 rotated fastest direction, the face hops with their periodic wrap and
-colours, every index inside [0, V) -- on every lattice and block grid the
+colours, the even-odd kernels' threads, compact indexes and hops, every index
+inside [0, V) -- on every lattice and block grid the
 GPU tests and the benchmark use, and on blocks one and two sites wide.
 A stand-in for a device bounds checker for the index arithmetic."""
 import shutil
@@ -30,6 +31,9 @@ GEOMETRIES = [
     "48,48,48,96/2,4,2,2", "48,48,48,96/2,1,1,1",
     # blocks one or two sites wide
     "8,4,4,4/8,4,4,4", "16,2,2,2/2,2,2,2", "4,4,4,4/4,2,2,2", "6,2,4,2/2,2,2,2",
+    # odd extents and rows of the even-odd tests, extents 2 and 3
+    "6,5,3,2/2,1,1,2", "6,5,3,2/2,1,1,1", "10,6,14,4/2,2,2,2", "10,3,3,3/2,1,1,1",
+    "4,2,2,4/2,1,1,1", "18,18,22,20/2,2,2,2",
 ]
 
 
@@ -58,5 +62,8 @@ def test_checker_catches_a_planted_mistake(checker):
     r = subprocess.run([str(checker), "planted:8,4,4,8/2,1,1,1"], capture_output=True, text=True,
                        timeout=60)
     assert r.returncode == 1 and r.stdout.startswith("FAIL"), r.stdout
+    r = subprocess.run([str(checker), "planted-eo:8,4,4,8/2,1,1,1"], capture_output=True, text=True,
+                       timeout=60)
+    assert r.returncode == 1 and r.stdout.startswith("FAIL pair"), r.stdout
     r = subprocess.run([str(checker), "8,8,8/2,1,1,1"], capture_output=True, text=True, timeout=60)
     assert r.returncode == 2 and "bad argument" in r.stdout
