@@ -47,14 +47,23 @@ __device__ __forceinline__ EoSite eo_site(const EoArgs<T>& a, int e) {
   return s;
 }
 
-// v: the neighbour's spinor (directions x, y, z) or its two spins (t); u: the
-// link.  acc += the hop's contribution
+// (the products are written out here and in eo_hop_planes: shared through a
+// function they came out with other register spills, mtilde in FP32 at 24^3x48
+// 169 -> 182 us)
 template <typename T, int DAG, int MU, int DIR, typename R = typename Arith<T>::R>
-__device__ __forceinline__ void eo_hop_with(const R u[18], const R v[24], bool t_edge, int tbc,
-                                            R acc[24]) {
+__device__ __forceinline__ void eo_hop(const EoArgs<T>& a, const EoSite& s, int e, R acc[24]) {
+  const int c = MU == 0 ? 2 * s.xh + s.odd : MU == 1 ? s.y : MU == 2 ? s.z : s.t;
+  const int en = eo_step(a.G, e, MU, DIR, c, s.xh, s.odd);
   constexpr int PD = DAG ? -DIR : DIR;  // projector / reconstruction of this hop
-  R h[12], r[12];
+  R v[24];
+  if (MU == 3)
+    IO<T>::load_half(a.src, a.pad, en, PD > 0, v);
+  else
+    IO<T>::load_spinor(a.src, a.pad, en, v);
+  R h[12], r[12], u[18];
   project<R, MU, PD>(v, h);
+  // forward: this parity's own link, backward: the other parity's
+  IO<T>::load_link(DIR > 0 ? a.U[0] : a.U[1], a.pad, MU, DIR > 0 ? e : en, u);
   if (DIR > 0)
     link_mul<R, false>(u, h, r);
   else
@@ -62,31 +71,16 @@ __device__ __forceinline__ void eo_hop_with(const R u[18], const R v[24], bool t
   R f = 1;
   if (MU == 3) {
     f = 2;
-    if (t_edge) f = (R)(2 * tbc);
+    if (DIR > 0 ? s.t == a.G.L[3] - 1 : s.t == 0) f = (R)(2 * a.G.tbc);
   }
   reconstruct<R, MU, PD>(r, acc, f);
-}
-
-template <typename T, int DAG, int MU, int DIR, typename R = typename Arith<T>::R>
-__device__ __forceinline__ void eo_hop(const EoArgs<T>& a, const EoSite& s, int e, R acc[24]) {
-  const int c = MU == 0 ? 0 : MU == 1 ? s.y : MU == 2 ? s.z : s.t;
-  const int en = eo_step(a.G, e, MU, DIR, c, s.xh, s.odd);
-  R v[24], u[18];
-  if (MU == 3)
-    IO<T>::load_half(a.src, a.pad, en, (DAG ? -DIR : DIR) > 0, v);
-  else
-    IO<T>::load_spinor(a.src, a.pad, en, v);
-  // forward: this parity's own link, backward: the other parity's
-  IO<T>::load_link(DIR > 0 ? a.U[0] : a.U[1], a.pad, MU, DIR > 0 ? e : en, u);
-  eo_hop_with<T, DAG, MU, DIR>(u, v, DIR > 0 ? s.t == a.G.L[3] - 1 : s.t == 0, a.G.tbc, acc);
 }
 
 // Memory bound: per output site 8 links (1152 bytes in FP64, each link of the
 // lattice once per launch), A^-1, the source once and the result: 2112 bytes
 // in FP64, 118 us at 24^3x48, 0.91 of the measured copy rate.
-// FP64 at 128 registers (4 CTAs of 128 threads an SM), FP32 at 80 (6)
 template <typename T, int DAG, int CLOV, int MODE>
-__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) k_eo(const EoArgs<T> a) {
+__device__ __forceinline__ void eo_body(const EoArgs<T>& a) {
   using R = typename Arith<T>::R;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= a.G.Vh) return;
@@ -111,6 +105,11 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) k_eo(const EoArgs
   }
   IO<T>::store_spinor(a.out, a.pad, e, acc);
 }
+// FP64 at 128 registers (4 CTAs of 128 threads an SM), FP32 at 80 (6)
+template <typename T, int DAG, int CLOV, int MODE>
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) k_eo(const EoArgs<T> a) {
+  eo_body<T, DAG, CLOV, MODE>(a);
+}
 
 // The same on the full planes.  Thread i takes the sites of parity pe among 2i
 // and 2i + 1 of the planes' order: one, where the two are neighbours along an
@@ -130,13 +129,25 @@ __device__ __forceinline__ void eo_hop_planes(const EoArgs<T>& a, const int x[4]
   int xn[4];
   eo_neighbour<MU, DIR>(a.G, x, a.pe, xn);
   const int gn = dd_index(a.G, xn);
+  constexpr int PD = DAG ? -DIR : DIR;
   R v[24], u[18];
   if (MU == 3)
-    IO<T>::load_half(a.src, a.G.pad, gn, (DAG ? -DIR : DIR) > 0, v);
+    IO<T>::load_half(a.src, a.G.pad, gn, PD > 0, v);
   else
     IO<T>::load_spinor(a.src, a.G.pad, gn, v);
   IO<T>::load_link(a.U[0], a.G.pad, MU, DIR > 0 ? g : gn, u);
-  eo_hop_with<T, DAG, MU, DIR>(u, v, DIR > 0 ? x[3] == a.G.L[3] - 1 : x[3] == 0, a.G.tbc, acc);
+  R h[12], r[12];
+  project<R, MU, PD>(v, h);
+  if (DIR > 0)
+    link_mul<R, false>(u, h, r);
+  else
+    link_mul<R, true>(u, h, r);
+  R f = 1;
+  if (MU == 3) {
+    f = 2;
+    if (DIR > 0 ? x[3] == a.G.L[3] - 1 : x[3] == 0) f = (R)(2 * a.G.tbc);
+  }
+  reconstruct<R, MU, PD>(r, acc, f);
 }
 template <typename T, int WHICH, int DAG, int CLOV, int MODE>
 __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) k_eo_planes(const EoArgs<T> a) {
